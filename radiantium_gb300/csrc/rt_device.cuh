@@ -379,8 +379,7 @@ struct Best {
 #define RT_TRAVERSAL_CAP (1u << 26)   /* loop steps of one two-level traversal */
 #endif
 #ifndef RT_DESCEND
-/* interior nodes one traversal step may visit in shallow trees (Cornell box / light tracer,
- * M samples / particles per s: 415 / 223 at 2, 421 / 229 at 3, 426 / 227 at 4, 418 / 224 at 5) */
+/* interior nodes a thread that traverses a ray alone visits between two LeafSteps */
 #define RT_DESCEND 3
 #endif
 #define RT_NO_NODE ((int)0x80000000)
@@ -579,42 +578,38 @@ DF int PopNext(Stk stack, int* sp, int base, float maxT, TravStats* st) {
     return RT_NO_NODE;
 }
 
-/* Leaf references become a primitive cursor (count in the first slot). */
-DF void EnterLeaf(const RtSceneView* S, int* cur, int* leafSlot, int* leafLeft) {
-    if (*cur != RT_NO_NODE && *cur < 0) {
-        *leafSlot = ~*cur;
-        *leafLeft = __float_as_int(__ldg(S->slots + 3 * (int64_t)*leafSlot + 2).w);
-        *cur = RT_NO_NODE;
-    }
-}
-
-/* Scene.Intersect(ray, out inct) over the two-level scene: Bvh.Intersect
- * (Accelerators/Bvh.cs:174-232) on the top-level tree and, for each instance
- * leaf, InstancedPrimitive.Intersect (Primitive.cs:169-188) on its prototype
- * tree in model space with world T = Distance(ray.O, p).  Boxes, MaxT culls
- * and primitive tests happen in exactly the order of the recursive form; the
- * recursion is unrolled into a state machine: a step visits up to kDescend
- * interior nodes (with the pops that follow them) and then, if that reached a
- * leaf, tests its next primitive, or leaves a prototype.  A lane that has just
- * reached a leaf tests it together with the lanes already in leaves, and rays
- * at different levels run the same step code together; a persistent kernel
- * can hand a lane a new ray between any two steps.  stack[0, base) holds
- * top-level entries, stack[base, base + RT_STACK_SIZE) the prototype's, so
- * `stack` has 2 * RT_STACK_SIZE entries. */
-struct TravClosest {
+/* Scene.Intersect over the two-level scene, in both forms: the closest hit
+ * (Bvh.Intersect(ray, out inct), Accelerators/Bvh.cs:174-232, and
+ * InstancedPrimitive.Intersect, Primitive.cs:169-188, with world
+ * T = Distance(ray.O, p)) and, kAny, the first hit found (Bvh.cs:126-172,
+ * Primitive.cs:162-167).  Boxes, MaxT culls and primitive tests happen in
+ * exactly the order of the recursive form; the recursion is unrolled into a
+ * state machine of two kinds of step, so that a warp can run the lanes that
+ * wait for the same kind together and hand a lane a new ray between any two:
+ *
+ *   DescendStep  visits one interior node, with the pops that follow it;
+ *   LeafStep     tests one primitive of a leaf, and enters or leaves an
+ *                instance's prototype.
+ *
+ * cur says which comes next: >= 0 an interior node to descend; < 0 a LeafStep
+ * (~cur is the first slot of a leaf just reached, or RT_NO_NODE: the next
+ * primitive of the leaf being tested, or the end of this level).
+ * stack[0, base) holds top-level entries, stack[base, base + RT_STACK_SIZE)
+ * the prototype's, so `stack` has 2 * RT_STACK_SIZE entries. */
+struct Traversal {
     Ray r;                       /* world ray, or the model-space ray inside a prototype */
     V3 wO, wD;                   /* the world ray */
     float wMaxT;                 /* the world ray's MaxT while a prototype is traversed */
     Best best;
     float pt, pu, pv; int pslot; uint32_t pflags;     /* the prototype's own closest hit */
     int cur, sp, base, leafSlot, leafLeft, topSlot, topLeft, inst;
-    bool any, inProto, pany;
+    bool any, inProto, pany;     /* kAny: `any` is the answer */
     uint32_t guard;
 };
 
 /* Returns true when the traversal is already over (empty scene or root box missed). */
 template <bool kWide = false>
-DF bool ClosestBegin(const RtSceneView* S, const Ray& ray, TravClosest& T, TravStats* st) {
+DF bool TraversalBegin(const RtSceneView* S, const Ray& ray, Traversal& T, TravStats* st) {
     Best& b = T.best;
     b.t = kFMax; b.flags = 0; b.slot = -1; b.sub = -1; b.u = 0; b.v = 0; b.pw = v3s(0);
     T.r = ray; T.wO = ray.O; T.wD = ray.D; T.wMaxT = ray.MaxT;
@@ -623,45 +618,48 @@ DF bool ClosestBegin(const RtSceneView* S, const Ray& ray, TravClosest& T, TravS
     T.pt = kFMax; T.pu = 0; T.pv = 0; T.pslot = -1; T.pflags = 0;
     T.guard = 0;
     T.cur = RootRef<kWide>(S, 0, ray, st);
-    if (T.cur == RT_NO_NODE) return true;
-    EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
+    return T.cur == RT_NO_NODE;
+}
+
+/* One interior node (T.cur >= 0); kWide: the fast traversal's wide nodes (a
+ * visit may push up to seven entries).  Returns true when the traversal has
+ * finished (a top-level stack overflow). */
+template <class Stk, bool kWide = false>
+DF bool DescendStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status, TravStats* st) {
+    if (kWide ? T.sp - T.base > RT_STACK_SIZE - 8 : T.sp - T.base == RT_STACK_SIZE) {
+        atomicOr(status, RT_STATUS_STACK);
+        T.cur = RT_NO_NODE;
+        if (!T.inProto) return true;
+        T.sp = T.base;                  /* the prototype's traversal stops here */
+        return false;
+    }
+    if (st) st->nodes++;
+    T.cur = kWide ? VisitWideNode(S, T.cur, T.r, stack, &T.sp) : VisitNode(S, T.cur, T.r, stack, &T.sp, st);
+    if (T.cur == RT_NO_NODE) T.cur = PopNext(stack, &T.sp, T.base, T.r.MaxT, st);
     return false;
 }
 
-/* One step; true when the traversal has finished.  kWide: the fast traversal's
- * wide nodes (a visit may push up to seven entries). */
-template <class Stk, int kDescend = RT_DESCEND, bool kWide = false>
-DF bool ClosestStep(const RtSceneView* S, TravClosest& T, Stk stack, uint32_t* status, TravStats* st) {
-    if (++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); return true; }
-    if (T.cur != RT_NO_NODE) {
-        /* up to kDescend interior nodes (with the pops that follow them) per step */
-        for (int k = 0; k < kDescend && T.cur >= 0; k++) {
-            if (kWide ? T.sp - T.base > RT_STACK_SIZE - 8 : T.sp - T.base == RT_STACK_SIZE) {
-                atomicOr(status, RT_STATUS_STACK);
-                if (!T.inProto) return true;
-                T.sp = T.base;                  /* the prototype's traversal stops here */
-                T.cur = RT_NO_NODE;
-                return false;
-            }
-            if (st) st->nodes++;
-            T.cur = kWide ? VisitWideNode(S, T.cur, T.r, stack, &T.sp) : VisitNode(S, T.cur, T.r, stack, &T.sp, st);
-            if (T.cur == RT_NO_NODE) T.cur = PopNext(stack, &T.sp, T.base, T.r.MaxT, st);
-        }
-        EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
-        if (T.cur != RT_NO_NODE) return false;      /* still descending: the next step goes on */
-    }
-    if (T.leafLeft > 0) {
-        const int slot = T.leafSlot++;
-        T.leafLeft--;
+/* One primitive, or the end of a level (T.cur < 0); true when the traversal has finished. */
+template <bool kAny, class Stk, bool kWide = false>
+DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status, TravStats* st) {
+    const bool fresh = T.cur != RT_NO_NODE;
+    if (fresh || T.leafLeft > 0) {
+        const int slot = fresh ? ~T.cur : T.leafSlot;
         const float4 s0 = __ldg(S->slots + 3 * (int64_t)slot);
         const float4 s1 = __ldg(S->slots + 3 * (int64_t)slot + 1);
         const float4 s2 = __ldg(S->slots + 3 * (int64_t)slot + 2);
+        T.leafSlot = slot + 1;
+        T.leafLeft = (fresh ? __float_as_int(s2.w) : T.leafLeft) - 1;    /* a leaf's count is in its first slot */
+        T.cur = RT_NO_NODE;
         const uint32_t kr = __float_as_uint(s1.w);
         const uint32_t kind = kr >> RT_KIND_SHIFT, ref = kr & RT_REF_MASK;
         if (st) st->prims++;
         if (kind != RT_KIND_INSTANCE) {
             float t, u, v;
             if (!PrimHit(S, kind, ref, s0, s1, s2, T.r, &t, &u, &v)) {
+            } else if (kAny) {
+                T.any = true;
+                return true;
             } else if (T.inProto) {
                 T.pany = true;
                 if (kWide && NearTie(t, T.pt)) T.pflags |= RT_HIT_TIE;
@@ -681,10 +679,7 @@ DF bool ClosestStep(const RtSceneView* S, TravClosest& T, Stk stack, uint32_t* s
             atomicOr(status, RT_STATUS_BADREF);
         }
         if (kind != RT_KIND_INSTANCE || T.inProto) {
-            if (T.leafLeft == 0) {
-                T.cur = PopNext(stack, &T.sp, T.base, T.r.MaxT, st);
-                EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
-            }
+            if (T.leafLeft == 0) T.cur = PopNext(stack, &T.sp, T.base, T.r.MaxT, st);
             return false;
         }
         /* enter the instance's prototype */
@@ -701,13 +696,12 @@ DF bool ClosestStep(const RtSceneView* S, TravClosest& T, Stk stack, uint32_t* s
         T.inProto = true;
         T.base = T.sp;
         T.cur = RootRef<kWide>(S, 1 + __ldg(&I.blas), T.r, st);
-        EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
         return false;
     }
     if (!T.inProto) return true;
     /* leave the prototype: the instance's candidate in world space */
     T.inProto = false;
-    if (T.pany) {
+    if (!kAny && T.pany) {
         const RtInstance& I = S->instances[T.inst];
         const float4 s1 = __ldg(S->slots + 3 * (int64_t)T.pslot + 1);
         const uint32_t kr = __float_as_uint(s1.w);
@@ -741,121 +735,37 @@ DF bool ClosestStep(const RtSceneView* S, TravClosest& T, Stk stack, uint32_t* s
     T.leafSlot = T.topSlot; T.leafLeft = T.topLeft;
     T.sp = T.base;
     T.base = 0;
-    if (T.leafLeft == 0) {
-        T.cur = PopNext(stack, &T.sp, 0, T.r.MaxT, st);
-        EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
-    }
+    if (T.leafLeft == 0) T.cur = PopNext(stack, &T.sp, 0, T.r.MaxT, st);
     return false;
 }
 
-/* The whole closest-hit traversal of one ray; ray.MaxT ends at the closest hit. */
+/* The whole traversal of one ray by one thread. */
+template <bool kAny, bool kWide = false>
+DF void Traverse(const RtSceneView* S, const Ray& ray, Traversal& T, int2* stack, uint32_t* status, TravStats* st) {
+    if (TraversalBegin<kWide>(S, ray, T, st)) return;
+    while (true) {
+        if (++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); return; }
+        for (int k = 0; k < RT_DESCEND && T.cur >= 0; k++)
+            if (DescendStep<int2*, kWide>(S, T, stack, status, st)) return;
+        if (T.cur < 0 && LeafStep<kAny, int2*, kWide>(S, T, stack, status, st)) return;
+    }
+}
+
+/* The closest hit of one ray; ray.MaxT ends at it. */
 template <bool kWide = false>
 DF bool SceneClosest(const RtSceneView* S, Ray& ray, Best* best, int2* stack, uint32_t* status, TravStats* st) {
-    TravClosest T;
-    if (!ClosestBegin<kWide>(S, ray, T, st))
-        while (!ClosestStep<int2*, RT_DESCEND, kWide>(S, T, stack, status, st)) {}
+    Traversal T;
+    Traverse<false, kWide>(S, ray, T, stack, status, st);
     *best = T.best;
     ray.MaxT = T.inProto ? T.wMaxT : T.r.MaxT;
     return T.any;
 }
 
-/* Scene.Intersect(ray): the any-hit form (Bvh.cs:126-172,
- * InstancedPrimitive.Intersect(ray), Primitive.cs:162-167). */
-struct TravAny {
-    Ray r;
-    V3 wO, wD;
-    float wMaxT;
-    int cur, sp, base, leafSlot, leafLeft, topSlot, topLeft;
-    bool inProto, hit;
-    uint32_t guard;
-};
-
-template <bool kWide = false>
-DF bool AnyBegin(const RtSceneView* S, const Ray& ray, TravAny& T, TravStats* st) {
-    T.r = ray; T.wO = ray.O; T.wD = ray.D; T.wMaxT = ray.MaxT;
-    T.inProto = false; T.hit = false;
-    T.base = 0; T.sp = 0; T.leafLeft = 0; T.leafSlot = 0; T.topSlot = 0; T.topLeft = 0;
-    T.guard = 0;
-    T.cur = RootRef<kWide>(S, 0, ray, st);
-    if (T.cur == RT_NO_NODE) return true;
-    EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
-    return false;
-}
-
-/* One step; true when the traversal has finished (T.hit holds the answer). */
-template <class Stk, int kDescend = RT_DESCEND, bool kWide = false>
-DF bool AnyStep(const RtSceneView* S, TravAny& T, Stk stack, uint32_t* status, TravStats* st) {
-    if (++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); return true; }
-    if (T.cur != RT_NO_NODE) {
-        for (int k = 0; k < kDescend && T.cur >= 0; k++) {
-            if (kWide ? T.sp - T.base > RT_STACK_SIZE - 8 : T.sp - T.base == RT_STACK_SIZE) {
-                atomicOr(status, RT_STATUS_STACK);
-                if (!T.inProto) return true;
-                T.sp = T.base;
-                T.cur = RT_NO_NODE;
-                return false;
-            }
-            if (st) st->nodes++;
-            T.cur = kWide ? VisitWideNode(S, T.cur, T.r, stack, &T.sp) : VisitNode(S, T.cur, T.r, stack, &T.sp, st);
-            if (T.cur == RT_NO_NODE) T.cur = PopNext(stack, &T.sp, T.base, T.r.MaxT, st);
-        }
-        EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
-        if (T.cur != RT_NO_NODE) return false;
-    }
-    if (T.leafLeft > 0) {
-        const int slot = T.leafSlot++;
-        T.leafLeft--;
-        const float4 s0 = __ldg(S->slots + 3 * (int64_t)slot);
-        const float4 s1 = __ldg(S->slots + 3 * (int64_t)slot + 1);
-        const float4 s2 = __ldg(S->slots + 3 * (int64_t)slot + 2);
-        const uint32_t kr = __float_as_uint(s1.w);
-        const uint32_t kind = kr >> RT_KIND_SHIFT, ref = kr & RT_REF_MASK;
-        if (st) st->prims++;
-        if (kind != RT_KIND_INSTANCE) {
-            float t, u, v;
-            if (PrimHit(S, kind, ref, s0, s1, s2, T.r, &t, &u, &v)) { T.hit = true; return true; }
-        } else if (T.inProto) {
-            atomicOr(status, RT_STATUS_BADREF);
-        }
-        if (kind != RT_KIND_INSTANCE || T.inProto) {
-            if (T.leafLeft == 0) {
-                T.cur = PopNext(stack, &T.sp, T.base, T.r.MaxT, st);
-                EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
-            }
-            return false;
-        }
-        if (st) st->insts++;
-        T.topSlot = T.leafSlot; T.topLeft = T.leafLeft; T.leafLeft = 0;
-        const RtInstance& I = S->instances[(int)ref];
-        float w2m[12];
-#pragma unroll
-        for (int i = 0; i < 12; i++) w2m[i] = __ldg(I.w2m + i);
-        T.r = XfRay(T.r, w2m);
-        T.inProto = true;
-        T.base = T.sp;
-        T.cur = RootRef<kWide>(S, 1 + __ldg(&I.blas), T.r, st);
-        EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
-        return false;
-    }
-    if (!T.inProto) return true;
-    T.inProto = false;
-    T.r = mkray(T.wO, T.wD, T.r.MinT, T.wMaxT);
-    T.leafSlot = T.topSlot; T.leafLeft = T.topLeft;
-    T.sp = T.base;
-    T.base = 0;
-    if (T.leafLeft == 0) {
-        T.cur = PopNext(stack, &T.sp, 0, T.r.MaxT, st);
-        EnterLeaf(S, &T.cur, &T.leafSlot, &T.leafLeft);
-    }
-    return false;
-}
-
 template <bool kWide = false>
 DF bool SceneAny(const RtSceneView* S, const Ray& ray, int2* stack, uint32_t* status, TravStats* st) {
-    TravAny T;
-    if (!AnyBegin<kWide>(S, ray, T, st))
-        while (!AnyStep<int2*, RT_DESCEND, kWide>(S, T, stack, status, st)) {}
-    return T.hit;
+    Traversal T;
+    Traverse<true, kWide>(S, ray, T, stack, status, st);
+    return T.any;
 }
 
 /* Builds the full Intersection of the winning primitive (GetIntersection /

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(256) k_wf_start(WfState W) {
  * keeps its lanes busy by handing a new queue entry to every lane whose ray
  * has finished, as soon as W.refill lanes are idle, instead of idling until
  * the warp's longest ray is done.  The traversal is the step machine of
- * TravClosest / TravAny, so a lane can take a new ray between any two steps
+ * Traversal, so a lane can take a new ray between any two steps
  * and the per-ray results are the same as a one-ray-per-thread launch. */
 constexpr unsigned kFullWarp = 0xffffffffu;
 
@@ -287,7 +287,7 @@ DF Ray queued_ray(const WfState& W, int q) {
     return mkray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, d.w);
 }
 
-DF void closest_done(const WfState& W, int meta, const TravClosest& T) {
+DF void closest_done(const WfState& W, int meta, const Traversal& T) {
     const int path = meta_path(meta);
     const float4 h = make_float4(T.best.t, T.best.u, T.best.v, __int_as_float(T.any ? T.best.slot : -1));
     const int kind = meta_kind(meta);
@@ -295,12 +295,6 @@ DF void closest_done(const WfState& W, int meta, const TravClosest& T) {
     else if (kind == WF_RAY_MIS) { W.mis_hit[path] = h; W.mis_sub[path] = T.best.sub; }
     else { W.trw_hit[path] = h; W.trw_sub[path] = T.best.sub; }
 }
-
-/* interior nodes per traversal step in scenes with tall trees (C2 / C3 trace ms per step:
- * 85.7 / 24.3 at 3, 83.7 / 23.8 at 4, 83.5 / 23.7 at 5, 87.5 / 23.2 at 6) */
-#ifndef RT_DESCEND_DEEP
-#define RT_DESCEND_DEEP 5
-#endif
 
 /* The traversal stack of a trace kernel: with kSh (scenes with tall trees)
  * its bottom RT_SH_STACK entries live in shared memory, which keeps the stack
@@ -319,54 +313,6 @@ template <> struct TraceStack<true> {
     }
 };
 
-/* wide nodes per traversal step of the fast traversal (kWide) */
-#ifndef RT_DESCEND_WIDE
-#define RT_DESCEND_WIDE 1        /* C2 M samples/s: 154.7 at 1, 134.9 at 2, 120.5 at 3 */
-#endif
-
-/* closest-hit rays: extension and MIS rays (queue [0, n_closest)); kWide: the
- * opt-in fast traversal over the wide nodes */
-template <bool kSh, bool kWide>
-__global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_CLOSEST_BLOCKS) k_wf_trace_closest(WfState W, uint32_t* status, unsigned long long* stats,
-                                                            bool counting) {
-    const int n = min(W.ctr->n_closest, 2 * W.slots);
-    TraceStack<kSh> stk;
-    const auto stack = stk.get();
-    TravStats st = {0, 0, 0};
-    TravStats* pst = counting ? &st : nullptr;
-    uint32_t done = 0;
-    TravClosest T;
-    const RtSceneView* S = nullptr;
-    int item = -1, meta = 0;
-    bool exhausted = false;
-    while (true) {
-        const unsigned idle = __ballot_sync(kFullWarp, item < 0);
-        if (exhausted) {
-            if (idle == kFullWarp) break;
-        } else if (__popc(idle) >= W.refill) {
-            const int q = fetch_entry(&W.ctr->fetch[0], n, idle, &exhausted);
-            if (item < 0 && q < n) {
-                meta = W.q_meta[q];
-                S = W.jobs[meta_job(meta)].view;
-                if (ClosestBegin<kWide>(S, queued_ray(W, q), T, pst)) { closest_done(W, meta, T); done++; }
-                else item = q;
-            }
-        }
-        if (item >= 0 && ClosestStep<decltype(stack), kWide ? RT_DESCEND_WIDE : (kSh ? RT_DESCEND_DEEP : RT_DESCEND), kWide>(
-                             S, T, stack, status, pst)) {
-            closest_done(W, meta, T);
-            done++;
-            item = -1;
-        }
-    }
-    if (counting) {
-        warp_add64(stats + 1, done);
-        warp_add64(stats + 3, st.nodes);
-        warp_add64(stats + 4, st.prims);
-        warp_add64(stats + 5, st.insts);
-    }
-}
-
 /* a shadow ray's answer: the path's occlusion flag, or for a light-tracer
  * camera connection its splat, added to the film sums when nothing is in the
  * way (the reference's `lock (renderTarget)` add, AdjointParticleIntegrator.cs:53-66) */
@@ -381,47 +327,104 @@ DF void shadow_done(const WfState& W, int meta, bool hit) {
         atomicAdd(reinterpret_cast<float4*>(J.samples) + pix, make_float4(sp.x, sp.y, sp.z, 0.0f));
 }
 
-/* shadow rays: any-hit (queue [shadow_base, shadow_base + n_shadow)) */
-template <bool kSh, bool kWide>
-__global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_SHADOW_BLOCKS) k_wf_trace_shadow(WfState W, uint32_t* status, unsigned long long* stats,
-                                                           bool counting) {
-    const int n = min(W.ctr->n_shadow, W.slots);
+
+/* When a warp stops descending: as soon as this many of 32 live lanes wait for
+ * a LeafStep (a share of the live lanes when fewer are live).  A low count
+ * runs the leaf, instance-entry and instance-exit code for few lanes at a
+ * time, a high one lets the lanes that reached a leaf idle; deep trees reach
+ * leaves less often, so they wait less.  Trace ms of a 64-spp Cornell frame
+ * (5-level tree) at 12 / 16 / 20 / 24: 3.70 / 3.58 / 3.53 / 3.52, against 3.73
+ * with up to three nodes and one leaf per step; of a 16-spp pass over the
+ * 64 x 200 k-triangle instances at 4 / 8 / 12 / 14 / 16 / 20: 82.7 / 76.3 /
+ * 73.1 / 72.8 / 72.7 / 75.3, against 79.6 with up to five nodes per step. */
+#ifndef RT_LEAF_WAIT
+#define RT_LEAF_WAIT 22          /* shallow trees */
+#endif
+#ifndef RT_LEAF_WAIT_DEEP
+#define RT_LEAF_WAIT_DEEP 14     /* trees of RT_DEEP_TREE levels and more */
+#endif
+/* nodes a lane may visit in one run before the warp's fetch check (8 to 64 measured alike) */
+#ifndef RT_DESCEND_RUN
+#define RT_DESCEND_RUN 16
+#endif
+
+/* The persistent traversal of one ray queue: entries [first, first + n), handed
+ * out by *counter.  Bound by lane utilisation and by the latency of dependent
+ * node loads (the tree sits in L2): lanes at nodes, leaves and instance
+ * boundaries would otherwise run one after another in every step, so the warp
+ * runs one kind at a time for all lanes that wait for it. */
+template <bool kAny, bool kSh, bool kWide>
+DF void trace_queue(const WfState& W, int first, int n, int32_t* counter, uint32_t* status, unsigned long long* stats,
+                    bool counting) {
     TraceStack<kSh> stk;
     const auto stack = stk.get();
+    typedef decltype(stk.get()) Stk;
     TravStats st = {0, 0, 0};
     TravStats* pst = counting ? &st : nullptr;
     uint32_t done = 0;
-    TravAny T;
+    Traversal T;
+    T.cur = RT_NO_NODE;
     const RtSceneView* S = nullptr;
     int item = -1, meta = 0;
     bool exhausted = false;
     while (true) {
-        const unsigned idle = __ballot_sync(kFullWarp, item < 0);
+        const unsigned busy = __ballot_sync(kFullWarp, item >= 0);
         if (exhausted) {
-            if (idle == kFullWarp) break;
-        } else if (__popc(idle) >= W.refill) {
-            const int e = fetch_entry(&W.ctr->fetch[1], n, idle, &exhausted);
-            if (item < 0 && e < n) {
-                const int q = W.shadow_base + e;
-                meta = W.q_meta[q];
+            if (!busy) break;
+        } else if (32 - __popc(busy) >= W.refill) {
+            const int q = fetch_entry(counter, n, ~busy, &exhausted);
+            if (item < 0 && q < n) {
+                item = first + q;
+                meta = W.q_meta[item];
                 S = W.jobs[meta_job(meta)].view;
-                if (AnyBegin<kWide>(S, queued_ray(W, q), T, pst)) { shadow_done(W, meta, false); done++; }
-                else item = q;
+                if (TraversalBegin<kWide>(S, queued_ray(W, item), T, pst)) {
+                    if (kAny) shadow_done(W, meta, false); else closest_done(W, meta, T);
+                    done++;
+                    item = -1;
+                    T.cur = RT_NO_NODE;
+                }
             }
         }
-        if (item >= 0 && AnyStep<decltype(stack), kWide ? RT_DESCEND_WIDE : (kSh ? RT_DESCEND_DEEP : RT_DESCEND), kWide>(
-                             S, T, stack, status, pst)) {
-            shadow_done(W, meta, T.hit);
-            done++;
-            item = -1;
+        bool over = false;
+        if (item >= 0 && ++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); over = true; T.cur = RT_NO_NODE; }
+        const int live = __popc(__ballot_sync(kFullWarp, item >= 0 && !over));
+        const int wait = (live * (kSh ? RT_LEAF_WAIT_DEEP : RT_LEAF_WAIT) + 31) >> 5;
+#pragma unroll 1
+        for (int k = 0; k < RT_DESCEND_RUN; k++) {
+            if (T.cur >= 0 && DescendStep<Stk, kWide>(S, T, stack, status, pst)) over = true;
+            if (live - __popc(__ballot_sync(kFullWarp, T.cur >= 0)) >= wait) break;
+        }
+        if (item >= 0 && T.cur < 0) {
+            if (over || LeafStep<kAny, Stk, kWide>(S, T, stack, status, pst)) {
+                if (kAny) shadow_done(W, meta, T.any); else closest_done(W, meta, T);
+                done++;
+                item = -1;
+                T.cur = RT_NO_NODE;
+            }
         }
     }
     if (counting) {
-        warp_add64(stats + 2, done);
+        warp_add64(stats + (kAny ? 2 : 1), done);
         warp_add64(stats + 3, st.nodes);
         warp_add64(stats + 4, st.prims);
         warp_add64(stats + 5, st.insts);
     }
+}
+
+/* closest-hit rays: extension and MIS rays (queue [0, n_closest)); kWide: the
+ * opt-in fast traversal over the wide nodes */
+template <bool kSh, bool kWide>
+__global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_CLOSEST_BLOCKS) k_wf_trace_closest(WfState W, uint32_t* status, unsigned long long* stats,
+                                                            bool counting) {
+    trace_queue<false, kSh, kWide>(W, 0, min(W.ctr->n_closest, 2 * W.slots), &W.ctr->fetch[0], status, stats, counting);
+}
+
+/* shadow rays: any-hit (queue [shadow_base, shadow_base + n_shadow)) */
+template <bool kSh, bool kWide>
+__global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_SHADOW_BLOCKS) k_wf_trace_shadow(WfState W, uint32_t* status, unsigned long long* stats,
+                                                           bool counting) {
+    trace_queue<true, kSh, kWide>(W, W.shadow_base, min(W.ctr->n_shadow, W.slots), &W.ctr->fetch[1], status, stats,
+                                  counting);
 }
 
 DF bool load_hit(const RtSceneView* S, const Ray& ray, float4 h, int sub, Isect* it) {
