@@ -396,7 +396,14 @@ int emit_wide(const rtb::BuildResult& br, int slot_base, std::vector<float4>& wn
     return w.max_push;
 }
 
-void emit_bvh(const rtb::BuildResult& br, const std::vector<std::array<float4, 3>>& recs, std::vector<float4>& nodes,
+/* a box with min > max on an axis (a sphere of negative radius): the short
+ * form of the slab test does not hold for it */
+bool inverted(const rtb::Box& b) {
+    return b.mn[0] > b.mx[0] || b.mn[1] > b.mx[1] || b.mn[2] > b.mx[2];
+}
+
+/* returns whether a box is inverted */
+bool emit_bvh(const rtb::BuildResult& br, const std::vector<std::array<float4, 3>>& recs, std::vector<float4>& nodes,
               std::vector<float4>& slots, RtBvh* hdr) {
     const int slot_base = (int)(slots.size() / 3);
     for (size_t i = 0; i < br.order.size(); i++) {
@@ -407,8 +414,9 @@ void emit_bvh(const rtb::BuildResult& br, const std::vector<std::array<float4, 3
     if (fn.empty()) {
         for (int k = 0; k < 3; k++) { hdr->root_min[k] = 0; hdr->root_max[k] = 0; }
         hdr->root_ref = INT_MIN;
-        return;
+        return false;
     }
+    bool odd = inverted(fn[0].bounds);
     /* interior nodes get consecutive device indices in depth-first order */
     std::vector<int> dev(fn.size(), -1);
     int node_base = (int)(nodes.size() / 4), nint = 0;
@@ -428,14 +436,16 @@ void emit_bvh(const rtb::BuildResult& br, const std::vector<std::array<float4, 3
         if (fn[i].count != 0) { ref_of((int)i); continue; }
         const rtb::Box& L = fn[i + 1].bounds;
         const rtb::Box& R = fn[fn[i].second].bounds;
+        odd = odd || inverted(L) || inverted(R);
         int lref = ref_of((int)i + 1), rref = ref_of(fn[i].second), axis = fn[i].axis;
-        float4 n0 = make_float4(L.mn[0], L.mn[1], L.mn[2], L.mx[0]);
-        float4 n1 = make_float4(L.mx[1], L.mx[2], R.mn[0], R.mn[1]);
-        float4 n2 = make_float4(R.mn[2], R.mx[0], R.mx[1], R.mx[2]);
+        float4 n0 = make_float4(L.mn[0], R.mn[0], L.mx[0], R.mx[0]);
+        float4 n1 = make_float4(L.mn[1], R.mn[1], L.mx[1], R.mx[1]);
+        float4 n2 = make_float4(L.mn[2], R.mn[2], L.mx[2], R.mx[2]);
         float4 n3;
         std::memcpy(&n3.x, &lref, 4); std::memcpy(&n3.y, &rref, 4); std::memcpy(&n3.z, &axis, 4); n3.w = 0;
         nodes.push_back(n0); nodes.push_back(n1); nodes.push_back(n2); nodes.push_back(n3);
     }
+    return odd;
 }
 
 inline float4 f4bits(float x, float y, float z, int w) { float4 r = make_float4(x, y, z, 0); std::memcpy(&r.w, &w, 4); return r; }
@@ -534,6 +544,7 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
 
     std::vector<float4> nodes, slots, wnodes;
     int wide_push = 0;
+    bool odd_boxes = false;                    /* a box with min > max */
     std::vector<RtBvh> bvhs(1 + d->blas_count);
     /* instanced prototypes: ShapeWrapperPrimitive per shape (RendererBuilder.cs:895-921) */
     std::vector<rtb::Box> blas_root(d->blas_count);
@@ -562,7 +573,7 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
         rtb::BuildResult br = build_tree(c, boxes, maxp, threads);
         tallest = std::max(tallest, br.max_depth);
         const int blas_slots = (int)(slots.size() / 3);
-        emit_bvh(br, recs, nodes, slots, &bvhs[1 + b]);
+        odd_boxes = emit_bvh(br, recs, nodes, slots, &bvhs[1 + b]) || odd_boxes;
         wide_push = std::max(wide_push, emit_wide(br, blas_slots, wnodes, &bvhs[1 + b]));
         if (!br.nodes.empty()) blas_root[b] = br.nodes[0].bounds;
         else blas_root[b] = rtb::empty_box();
@@ -649,7 +660,7 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
     rtb::BuildResult top = build_tree(c, boxes, maxp, threads);
     tallest = std::max(tallest, top.max_depth);
     const int top_slots = (int)(slots.size() / 3);
-    emit_bvh(top, recs, nodes, slots, &bvhs[0]);
+    odd_boxes = emit_bvh(top, recs, nodes, slots, &bvhs[0]) || odd_boxes;
     wide_push = std::max(wide_push, emit_wide(top, top_slots, wnodes, &bvhs[0]));
 
     /* textures */
@@ -773,12 +784,13 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
     v.light_count = (int)lights.size();
     v.infinite_count = (int)infinite.size();
     v.global_medium = d->global_medium < 0 ? -1 : d->global_medium;
-    v.deep_trees = tallest > RT_STACK_SIZE + 1 ? 1 : 0;
+    const bool overflows = tallest > RT_STACK_SIZE + 1;
+    v.general_trees = overflows || odd_boxes ? 1 : 0;
     c->tallest = tallest;
     if (wnodes.empty()) wnodes.push_back(make_float4(0, 0, 0, 0));
     v.wnodes = upload(c, wnodes);
     /* a wide visit pushes at most 7 entries on top of what is below it */
-    v.wide_ok = (!v.deep_trees && wide_push + 7 <= RT_STACK_SIZE) ? 1 : 0;
+    v.wide_ok = (!overflows && wide_push + 7 <= RT_STACK_SIZE) ? 1 : 0;
     RtCamera& cam = v.camera;
     cam.width = d->camera.width; cam.height = d->camera.height;
     cam.near_z = d->camera.near_z; cam.far_z = d->camera.far_z;
@@ -941,8 +953,8 @@ RtParams particle_params(Ctx* c, const rt_render_params* p, int64_t first, int64
     return P;
 }
 
-void ensure_wf_graph(Ctx* c, const WfState& W, bool vol, bool particle = false, bool sort = true, bool deep = false,
-                     bool wide = false);
+struct WfMode;
+void ensure_wf_graph(Ctx* c, const WfState& W, const WfMode& m);
 
 /* What a wavefront run shades, and how its kernels are chosen. */
 struct WfMode {
@@ -951,6 +963,7 @@ struct WfMode {
     bool sort = true;        /* regroup the active list by shade key before shading */
     bool deep = false;       /* trace kernels with the shared-memory stack (trees of 16+ levels) */
     bool wide = false;       /* the opt-in fast traversal over the wide nodes */
+    bool general = false;    /* a scene's trees need the general node visit */
 };
 /* CUDA-event times and launch counts of a run, summed over its rounds */
 struct WfTotals {
@@ -972,7 +985,7 @@ void wf_round(Ctx* c, const WfState& W, cudaStream_t s, bool use_graph, const Wf
     CK(rt_wf_start(W, s, m.particle));
     t->launches += 2;
     if (use_graph && pass == WF_PASS_RENDER) {
-        ensure_wf_graph(c, W, m.vol, m.particle, m.sort, m.deep, m.wide);
+        ensure_wf_graph(c, W, m);
         CK(cudaEventRecord(c->events[0], s));
         CK(cudaGraphLaunch(c->wf_exec, s));
         CK(cudaEventRecord(c->events[1], s));
@@ -993,7 +1006,7 @@ void wf_round(Ctx* c, const WfState& W, cudaStream_t s, bool use_graph, const Wf
         if (c->h_ctr->iter >= W.iter_cap) throw RtFail(RT_ERR_ITER_CAP, "wavefront: bounce iteration cap reached (WF_ITER_CAP)");
         NvtxRange nvtx_iter("rt.wavefront_iteration");
         CK(cudaEventRecord(c->events[0], s));
-        CK(rt_wf_trace(W, c->status, c->stats, c->counting, s, m.deep, m.wide, &c->fork));
+        CK(rt_wf_trace(W, c->status, c->stats, c->counting, s, m.deep, m.wide, m.general, &c->fork));
         CK(cudaEventRecord(c->events[1], s));
         CK(cudaEventRecord(c->events[2], s));
         CK(rt_wf_shade(W, c->h_ctr->n_active[c->h_ctr->iter & 1], c->status, c->stats, c->counting, 0, false, s,
@@ -1039,6 +1052,7 @@ void particle_wavefront(Ctx* c, const RtParams& P, int64_t first, int64_t count,
     m.sort = c->mat_types > 1;
     m.deep = c->tallest >= RT_DEEP_TREE;
     m.wide = c->traversal == RT_TRAVERSAL_WIDE && c->view.wide_ok;
+    m.general = c->view.general_trees != 0;
     WfTotals t;
     for (int64_t done = 0; done < count;) {
         if (c->cancel.load()) throw RtFail(RT_ERR_CANCELLED, "render cancelled");
@@ -1223,17 +1237,18 @@ struct WfJobIn {
     int mat_types;         /* distinct material types of the job's scene */
     int tallest;           /* levels of its tallest tree */
     bool wide_ok;          /* its wide trees fit the fast traversal's stack */
+    bool general;          /* its trees need the general node visit */
 };
 
 /* The bounce loop as a graph: a while node whose body is one iteration
  * (trace, phase, sort, shade, tail); the tail kernel clears the loop's
  * condition when no path is left.  Rebuilt when the path state moves or the
  * counting mode changes. */
-void ensure_wf_graph(Ctx* c, const WfState& W, bool vol, bool particle, bool sort, bool deep, bool wide) {
-    const uint64_t key = (c->wf_generation << 32) ^ ((uint64_t)wide << 63) ^ ((uint64_t)W.slots << 10) ^ ((uint64_t)deep << 9) ^
+void ensure_wf_graph(Ctx* c, const WfState& W, const WfMode& m) {
+    const uint64_t key = (c->wf_generation << 32) ^ ((uint64_t)m.wide << 63) ^ ((uint64_t)m.general << 62) ^ ((uint64_t)W.slots << 10) ^ ((uint64_t)m.deep << 9) ^
                          ((uint64_t)(uint32_t)W.iter_cap * 0x9E3779B97F4A7C15ull) ^
-                         ((uint64_t)sort << 8) ^ ((uint64_t)particle << 7) ^ ((uint64_t)W.refill << 2) ^
-                         ((uint64_t)vol << 1) ^ (c->counting ? 1u : 0u);
+                         ((uint64_t)m.sort << 8) ^ ((uint64_t)m.particle << 7) ^ ((uint64_t)W.refill << 2) ^
+                         ((uint64_t)m.vol << 1) ^ (c->counting ? 1u : 0u);
     if (c->wf_exec && c->wf_graph_key == key) return;
     if (c->wf_exec) { cudaGraphExecDestroy(c->wf_exec); c->wf_exec = nullptr; }
     if (c->wf_graph) { cudaGraphDestroy(c->wf_graph); c->wf_graph = nullptr; }
@@ -1250,9 +1265,9 @@ void ensure_wf_graph(Ctx* c, const WfState& W, bool vol, bool particle, bool sor
     cudaGraph_t body = np.conditional.phGraph_out[0];
     CK(cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     uint64_t launches = 0;
-    cudaError_t e1 = rt_wf_trace(W, c->status, c->stats, c->counting, c->stream, deep, wide, &c->fork);
+    cudaError_t e1 = rt_wf_trace(W, c->status, c->stats, c->counting, c->stream, m.deep, m.wide, m.general, &c->fork);
     cudaError_t e2 = rt_wf_shade(W, -1, c->status, c->stats, c->counting, loop, true, c->stream, &launches,
-                                 WF_PASS_RENDER, nullptr, vol, particle, sort);
+                                 WF_PASS_RENDER, nullptr, m.vol, m.particle, m.sort);
     cudaGraph_t captured = nullptr;
     CK(cudaStreamEndCapture(c->stream, &captured));
     CK(e1);
@@ -1286,6 +1301,7 @@ void wavefront_run(Ctx* c, const std::vector<WfJobIn>& jobs, cudaStream_t s, boo
     for (const WfJobIn& J : jobs) mode.deep = mode.deep || J.tallest >= RT_DEEP_TREE;
     mode.wide = c->traversal == RT_TRAVERSAL_WIDE;
     for (const WfJobIn& J : jobs) mode.wide = mode.wide && J.wide_ok;
+    for (const WfJobIn& J : jobs) mode.general = mode.general || J.general;
     ensure_events(c, 4);
     WfTotals tot;
     while (true) {
@@ -1358,6 +1374,7 @@ void render_wavefront(Ctx* c, RtParams P, int chunk, int64_t npix, cudaStream_t 
     jobs[0].mat_types = c->mat_types;
     jobs[0].tallest = c->tallest;
     jobs[0].wide_ok = c->view.wide_ok != 0;
+    jobs[0].general = c->view.general_trees != 0;
     /* AUTO drives vol_path's loop as a graph: its boundary walks make ~100 short iterations per
      * round, where the host loop's per-iteration synchronisation costs 9 % (C3) */
     const bool vol = P.integrator == RT_INTEGRATOR_VOL_PATH;
@@ -1399,6 +1416,7 @@ void render_batch(Ctx* c, const rt_batch_item* items, int n, bool device_out, cu
         jobs[i].mat_types = sc->mat_types;
         jobs[i].tallest = sc->tallest;
         jobs[i].wide_ok = sc->view.wide_ok != 0;
+        jobs[i].general = sc->view.general_trees != 0;
         film_off[i] = film_floats;
         film_floats += (int64_t)P.w * P.h * 3;
     }
@@ -1502,6 +1520,7 @@ void adjoint_backward(Ctx* c, const rt_render_params* p, const rt_adjoint_desc* 
         jobs[0].mat_types = c->mat_types;
         jobs[0].tallest = c->tallest;
         jobs[0].wide_ok = c->view.wide_ok != 0;
+    jobs[0].general = c->view.general_trees != 0;
         CK(cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), s));
         wavefront_run(c, jobs, s, false, &A);
         launches += c->last.kernel_launches;

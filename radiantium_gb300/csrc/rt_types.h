@@ -58,9 +58,9 @@ struct RtBvh {
 #define RT_WIDE_F4 6
 
 /* an interior node: float4 n0..n3
- *   n0 = (L.min.x, L.min.y, L.min.z, L.max.x)
- *   n1 = (L.max.y, L.max.z, R.min.x, R.min.y)
- *   n2 = (R.min.z, R.max.x, R.max.y, R.max.z)
+ *   n0 = (L.min.x, R.min.x, L.max.x, R.max.x)     left and right planes side by side, so the
+ *   n1 = (L.min.y, R.min.y, L.max.y, R.max.y)     slab test runs on packed pairs; two 32-byte
+ *   n2 = (L.min.z, R.min.z, L.max.z, R.max.z)     loads
  *   n3 = (int Lref, int Rref, int axis, 0)   refs: >= 0 node, < 0 ~first slot
  * a primitive slot: float4 s0..s2
  *   s0 = (Pa.xyz, int prim_id)            prim_id: index in the owner's primitive list
@@ -174,9 +174,10 @@ struct RtSceneView {
     int32_t light_count;
     int32_t infinite_count;
     int32_t global_medium;
-    int32_t deep_trees;         /* a tree is taller than RT_STACK_SIZE + 1 levels: its
-                                 * traversal may overflow the stack, so every far child
-                                 * is pushed exactly as the reference pushes it */
+    int32_t general_trees;      /* traversals visit nodes in the general form: a tree is taller
+                                 * than RT_STACK_SIZE + 1 levels (its traversal may overflow the
+                                 * stack, so every far child is pushed exactly as the reference
+                                 * pushes it), or a box has min > max (a negative sphere radius) */
     const float4* wnodes;       /* wide nodes of every tree (RT_WIDE_F4 float4 each) */
     int32_t wide_ok;            /* every wide traversal fits the stack: the fast mode may run */
     int32_t env_alias;          /* infinite lights pick texels from their alias tables */

@@ -353,9 +353,11 @@ DF void shadow_done(const WfState& W, int meta, bool hit) {
  * node loads (the tree sits in L2): lanes at nodes, leaves and instance
  * boundaries would otherwise run one after another in every step, so the warp
  * runs one kind at a time for all lanes that wait for it. */
-template <bool kAny, bool kSh, bool kWide>
+template <bool kAny, bool kSh, NodeMode kMode>
 DF void trace_queue(const WfState& W, int first, int n, int32_t* counter, uint32_t* status, unsigned long long* stats,
                     bool counting) {
+    constexpr bool kWide = kMode == kNodesWide;
+    if (kMode == kNodesShort) counting = false;
     TraceStack<kSh> stk;
     const auto stack = stk.get();
     typedef decltype(stk.get()) Stk;
@@ -391,7 +393,7 @@ DF void trace_queue(const WfState& W, int first, int n, int32_t* counter, uint32
         const int wait = (live * (kSh ? RT_LEAF_WAIT_DEEP : RT_LEAF_WAIT) + 31) >> 5;
 #pragma unroll 1
         for (int k = 0; k < RT_DESCEND_RUN; k++) {
-            if (T.cur >= 0 && DescendStep<Stk, kWide>(S, T, stack, status, pst)) over = true;
+            if (T.cur >= 0 && DescendStep<Stk, kMode>(T, stack, status, pst)) over = true;
             if (live - __popc(__ballot_sync(kFullWarp, T.cur >= 0)) >= wait) break;
         }
         if (item >= 0 && T.cur < 0) {
@@ -411,19 +413,18 @@ DF void trace_queue(const WfState& W, int first, int n, int32_t* counter, uint32
     }
 }
 
-/* closest-hit rays: extension and MIS rays (queue [0, n_closest)); kWide: the
- * opt-in fast traversal over the wide nodes */
-template <bool kSh, bool kWide>
+/* closest-hit rays: extension and MIS rays (queue [0, n_closest)) */
+template <bool kSh, NodeMode kMode>
 __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_CLOSEST_BLOCKS) k_wf_trace_closest(WfState W, uint32_t* status, unsigned long long* stats,
                                                             bool counting) {
-    trace_queue<false, kSh, kWide>(W, 0, min(W.ctr->n_closest, 2 * W.slots), &W.ctr->fetch[0], status, stats, counting);
+    trace_queue<false, kSh, kMode>(W, 0, min(W.ctr->n_closest, 2 * W.slots), &W.ctr->fetch[0], status, stats, counting);
 }
 
 /* shadow rays: any-hit (queue [shadow_base, shadow_base + n_shadow)) */
-template <bool kSh, bool kWide>
+template <bool kSh, NodeMode kMode>
 __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_SHADOW_BLOCKS) k_wf_trace_shadow(WfState W, uint32_t* status, unsigned long long* stats,
                                                            bool counting) {
-    trace_queue<true, kSh, kWide>(W, W.shadow_base, min(W.ctr->n_shadow, W.slots), &W.ctr->fetch[1], status, stats,
+    trace_queue<true, kSh, kMode>(W, W.shadow_base, min(W.ctr->n_shadow, W.slots), &W.ctr->fetch[1], status, stats,
                                   counting);
 }
 
@@ -1606,38 +1607,47 @@ cudaError_t rt_wf_start(const WfState& W, cudaStream_t s, bool particle) {
     return cudaGetLastError();
 }
 
+namespace {
+
+typedef void (*TraceKernel)(WfState, uint32_t*, unsigned long long*, bool);
+/* the trace kernels by [node mode][shared-memory stack] */
+const TraceKernel kClosest[3][2] = {
+    {k_wf_trace_closest<false, kNodesGeneral>, k_wf_trace_closest<true, kNodesGeneral>},
+    {k_wf_trace_closest<false, kNodesShort>, k_wf_trace_closest<true, kNodesShort>},
+    {k_wf_trace_closest<false, kNodesWide>, k_wf_trace_closest<true, kNodesWide>}};
+const TraceKernel kShadow[3][2] = {
+    {k_wf_trace_shadow<false, kNodesGeneral>, k_wf_trace_shadow<true, kNodesGeneral>},
+    {k_wf_trace_shadow<false, kNodesShort>, k_wf_trace_shadow<true, kNodesShort>},
+    {k_wf_trace_shadow<false, kNodesWide>, k_wf_trace_shadow<true, kNodesWide>}};
+
+/* resident blocks of every trace kernel */
+struct TraceGrids {
+    int closest[3][2], shadow[3][2];
+    TraceGrids() {
+        for (int m = 0; m < 3; m++)
+            for (int d = 0; d < 2; d++) {
+                closest[m][d] = resident_blocks(kClosest[m][d], RT_TRACE_BLOCK);
+                shadow[m][d] = resident_blocks(kShadow[m][d], RT_TRACE_BLOCK);
+            }
+    }
+};
+
+}  // namespace
+
 cudaError_t rt_wf_trace(const WfState& W, uint32_t* status, unsigned long long* stats, bool counting, cudaStream_t s,
-                        bool deep, bool wide, const WfFork* fork) {
-    static const int closest_blocks[4] = {resident_blocks(k_wf_trace_closest<false, false>, RT_TRACE_BLOCK),
-                                          resident_blocks(k_wf_trace_closest<true, false>, RT_TRACE_BLOCK),
-                                          resident_blocks(k_wf_trace_closest<false, true>, RT_TRACE_BLOCK),
-                                          resident_blocks(k_wf_trace_closest<true, true>, RT_TRACE_BLOCK)};
-    static const int shadow_blocks[4] = {resident_blocks(k_wf_trace_shadow<false, false>, RT_TRACE_BLOCK),
-                                         resident_blocks(k_wf_trace_shadow<true, false>, RT_TRACE_BLOCK),
-                                         resident_blocks(k_wf_trace_shadow<false, true>, RT_TRACE_BLOCK),
-                                         resident_blocks(k_wf_trace_shadow<true, true>, RT_TRACE_BLOCK)};
-    const int v = (deep ? 1 : 0) + (wide ? 2 : 0);
+                        bool deep, bool wide, bool general, const WfFork* fork) {
+    static const TraceGrids grids;
+    const int m = wide ? kNodesWide : (general || counting ? kNodesGeneral : kNodesShort), d = deep ? 1 : 0;
     cudaError_t e = cudaSuccess;
     if (fork) {
         e = cudaEventRecord(fork->fork, s);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(fork->side, fork->fork, 0);
         if (e != cudaSuccess) return e;
     }
-    switch (v) {
-    case 0: k_wf_trace_closest<false, false><<<closest_blocks[0], RT_TRACE_BLOCK, 0, s>>>(W, status, stats, counting); break;
-    case 1: k_wf_trace_closest<true, false><<<closest_blocks[1], RT_TRACE_BLOCK, 0, s>>>(W, status, stats, counting); break;
-    case 2: k_wf_trace_closest<false, true><<<closest_blocks[2], RT_TRACE_BLOCK, 0, s>>>(W, status, stats, counting); break;
-    default: k_wf_trace_closest<true, true><<<closest_blocks[3], RT_TRACE_BLOCK, 0, s>>>(W, status, stats, counting); break;
-    }
+    kClosest[m][d]<<<grids.closest[m][d], RT_TRACE_BLOCK, 0, s>>>(W, status, stats, counting);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const cudaStream_t ss = fork ? fork->side : s;
-    switch (v) {
-    case 0: k_wf_trace_shadow<false, false><<<shadow_blocks[0], RT_TRACE_BLOCK, 0, ss>>>(W, status, stats, counting); break;
-    case 1: k_wf_trace_shadow<true, false><<<shadow_blocks[1], RT_TRACE_BLOCK, 0, ss>>>(W, status, stats, counting); break;
-    case 2: k_wf_trace_shadow<false, true><<<shadow_blocks[2], RT_TRACE_BLOCK, 0, ss>>>(W, status, stats, counting); break;
-    default: k_wf_trace_shadow<true, true><<<shadow_blocks[3], RT_TRACE_BLOCK, 0, ss>>>(W, status, stats, counting); break;
-    }
+    kShadow[m][d]<<<grids.shadow[m][d], RT_TRACE_BLOCK, 0, fork ? fork->side : s>>>(W, status, stats, counting);
     e = cudaGetLastError();
     if (e != cudaSuccess || !fork) return e;
     e = cudaEventRecord(fork->join, fork->side);

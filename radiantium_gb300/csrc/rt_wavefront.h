@@ -130,7 +130,8 @@ cudaError_t rt_wf_start(const WfState& W, cudaStream_t s, bool particle = false)
 /* Traces the queued closest-hit and shadow rays (lengths read on the device);
  * `deep`: a tree of the scene has RT_DEEP_TREE levels or more, the kernels
  * keep the bottom of the traversal stack in shared memory.  `wide`: the
- * opt-in fast traversal over the scenes' wide nodes. */
+ * opt-in fast traversal over the scenes' wide nodes.  `general`: a scene has
+ * RtSceneView::general_trees (counting runs use the general form too). */
 #ifndef RT_DEEP_TREE
 #define RT_DEEP_TREE 16
 #endif
@@ -143,7 +144,7 @@ struct WfFork {
     cudaEvent_t fork, join;
 };
 cudaError_t rt_wf_trace(const WfState& W, uint32_t* status, unsigned long long* stats, bool counting, cudaStream_t s,
-                        bool deep = false, bool wide = false, const WfFork* fork = nullptr);
+                        bool deep = false, bool wide = false, bool general = false, const WfFork* fork = nullptr);
 /* Shades the active paths (`particle`: light-tracer particles) - regrouped by
  * shade key first with `sort` - then advances the iteration; with `loop` set
  * (inside a captured while-loop), also sets the loop's condition to "paths
