@@ -91,6 +91,25 @@ RT_DM_FN float rt_dm_pow2i(int k) { return rt_dm_u2f((uint32_t)(k + 127) << 23);
 #define RT_DM_PIO2_4 2.5633440682570896e-12f
 #define RT_DM_2_OVER_PI 0.6366197466850281f
 
+/* The reduction of a large argument, in binary64 (IEEE, identical everywhere).
+ * Out of line on the device: callers' angles are small, and inlined copies of
+ * it only fill the shading kernels' instruction cache. */
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__
+#else
+static inline
+#endif
+float rt_dm_reduce_large(float x, int* q) {
+    double xd = (double)x;
+    double kd = xd * 0.63661977236758134308;
+    double kr = (kd >= 0.0) ? (double)(int64_t)(kd + 0.5) : -(double)(int64_t)(-kd + 0.5);
+    double r = xd - kr * 1.5707963267341256;
+    r = r - kr * 6.077100506506192e-11;
+    r = r - kr * 2.0222662487959506e-21;
+    int64_t ki = (int64_t)kr;
+    *q = (int)(ki & 3);
+    return (float)r;
+}
 /* Reduce x to r in [-pi/4, pi/4] (approximately) and quadrant q (0..3). */
 RT_DM_FN float rt_dm_reduce_pio2(float x, int* q) {
     float ax = x < 0.0f ? -x : x;
@@ -104,16 +123,10 @@ RT_DM_FN float rt_dm_reduce_pio2(float x, int* q) {
         *q = ki & 3;
         return r;
     }
-    /* large arguments: reduction in binary64 (IEEE, identical everywhere) */
-    double xd = (double)x;
-    double kd = xd * 0.63661977236758134308;
-    double kr = (kd >= 0.0) ? (double)(int64_t)(kd + 0.5) : -(double)(int64_t)(-kd + 0.5);
-    double r = xd - kr * 1.5707963267341256;
-    r = r - kr * 6.077100506506192e-11;
-    r = r - kr * 2.0222662487959506e-21;
-    int64_t ki = (int64_t)kr;
-    *q = (int)(ki & 3);
-    return (float)r;
+    int large;
+    float r = rt_dm_reduce_large(x, &large);
+    *q = large;
+    return r;
 }
 RT_DM_FN float rt_dm_sin_poly(float r) {
     float r2 = r * r;
@@ -135,28 +148,24 @@ RT_DM_FN float rt_dm_cos_poly(float r) {
     float tail = ((1.0f - w) - hr) + (r2 * r2) * p;
     return w + tail;
 }
-RT_DM_FN float rt_sinf(float x) {
-    if (rt_dm_isnan(x) || rt_dm_isinf(x)) return rt_dm_qnan();
+/* sine and cosine of one angle: one reduction, both polynomials, and the
+ * quadrant's pick without a branch (a warp's lanes sit in different quadrants) */
+RT_DM_FN void rt_sincosf(float x, float* s, float* c) {
+    if (rt_dm_isnan(x) || rt_dm_isinf(x)) { *s = rt_dm_qnan(); *c = rt_dm_qnan(); return; }
     int q; float r = rt_dm_reduce_pio2(x, &q);
-    float s;
-    switch (q) {
-        case 0: s = rt_dm_sin_poly(r); break;
-        case 1: s = rt_dm_cos_poly(r); break;
-        case 2: s = -rt_dm_sin_poly(r); break;
-        default: s = -rt_dm_cos_poly(r); break;
-    }
+    float sp = rt_dm_sin_poly(r), cp = rt_dm_cos_poly(r);
+    float a = (q & 1) ? cp : sp, b = (q & 1) ? sp : cp;
+    *s = (q & 2) ? -a : a;
+    *c = ((q + 1) & 2) ? -b : b;
+}
+RT_DM_FN float rt_sinf(float x) {
+    float s, c;
+    rt_sincosf(x, &s, &c);
     return s;
 }
 RT_DM_FN float rt_cosf(float x) {
-    if (rt_dm_isnan(x) || rt_dm_isinf(x)) return rt_dm_qnan();
-    int q; float r = rt_dm_reduce_pio2(x, &q);
-    float c;
-    switch (q) {
-        case 0: c = rt_dm_cos_poly(r); break;
-        case 1: c = -rt_dm_sin_poly(r); break;
-        case 2: c = -rt_dm_cos_poly(r); break;
-        default: c = rt_dm_sin_poly(r); break;
-    }
+    float s, c;
+    rt_sincosf(x, &s, &c);
     return c;
 }
 RT_DM_FN float rt_tanf(float x) {

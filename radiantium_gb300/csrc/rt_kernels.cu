@@ -139,6 +139,7 @@ __global__ void k_detmath(int fn, const float* a, const float* b, float* out, in
     case 5: r = rt_acosf(x); break;
     case 6: r = rt_expf(x); break;
     case 7: r = rt_logf(x); break;
+    case 8: r = PowerHeuristic(x, y); break;
     case 100: r = sinf(x); break;
     case 101: r = cosf(x); break;
     case 102: r = tanf(x); break;

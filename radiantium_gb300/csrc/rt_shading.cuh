@@ -13,7 +13,6 @@
 
 namespace rtd {
 
-#define NF static __device__ __noinline__
 
 /* the scene services share one traversal context per path */
 struct Ctx {
@@ -92,7 +91,8 @@ DF V3 DistSampleWh(const Dist& d, V3 wo, Rng& rand) {
             float logSample = rt_logf(1 - u.x);
             phi = rt_atanf(d.ay / d.ax * rt_tanf(2 * kPI * u.y + 0.5f * kPI));
             if (u.y > 0.5f) phi += kPI;
-            float sinPhi = rt_sinf(phi), cosPhi = rt_cosf(phi);
+            float sinPhi, cosPhi;
+            rt_sincosf(phi, &sinPhi, &cosPhi);
             float ax2 = d.ax * d.ax, ay2 = d.ay * d.ay;
             tan2Theta = -logSample / (cosPhi * cosPhi / ax2 + sinPhi * sinPhi / ay2);
         }
@@ -111,7 +111,8 @@ DF V3 DistSampleWh(const Dist& d, V3 wo, Rng& rand) {
     } else {
         phi = rt_atanf(d.ay / d.ax * rt_tanf(2 * kPI * u.y + .5f * kPI));
         if (u.y > 0.5f) phi += kPI;
-        float sinPhi = rt_sinf(phi), cosPhi = rt_cosf(phi);
+        float sinPhi, cosPhi;
+        rt_sincosf(phi, &sinPhi, &cosPhi);
         float ax2 = d.ax * d.ax, ay2 = d.ay * d.ay;
         float alpha2 = 1 / (cosPhi * cosPhi / ax2 + sinPhi * sinPhi / ay2);
         float tanTheta2 = alpha2 * u.x / (1 - u.x);
@@ -482,7 +483,8 @@ DF float MedSampleWi(const RtMedium& m, V3 wo, Rng& rand, V3* wiOut) {
     float sinTheta = Sqrt(nmax(0, 1 - cosTheta * cosTheta));
     float phi = 2 * kPI * rng.y;
     Frame f = mkframe(wo);
-    float sinPhi = rt_sinf(phi), cosPhi = rt_cosf(phi);
+    float sinPhi, cosPhi;
+    rt_sincosf(phi, &sinPhi, &cosPhi);
     *wiOut = sinTheta * cosPhi * f.X + sinTheta * sinPhi * f.Y + cosTheta * f.Z;
     return HGValue(cosTheta, g);
 }
@@ -621,11 +623,12 @@ NF LSample LightSampleLi(const RtSceneView* S, int li, V3 refP, Rng& rand) {
         float x = (float)ou / (float)d.nu;
         float theta = y * kPI;
         float phi = x * 2 * kPI;
-        float sinTheta = rt_sinf(theta);
+        float sinTheta, cosTheta;
+        rt_sincosf(theta, &sinTheta, &cosTheta);
         if (sinTheta == 0) return r;
         pdf /= (2 * kPI * kPI * sinTheta);
-        float cosTheta = rt_cosf(theta);
-        float sinPhi = rt_sinf(phi), cosPhi = rt_cosf(phi);
+        float sinPhi, cosPhi;
+        rt_sincosf(phi, &sinPhi, &cosPhi);
         V3 sph = v3(cosPhi * sinTheta, sinPhi * sinTheta, cosTheta);
         V3 dir = v3(sph.y, sph.z, -sph.x);
         V3 worldDir = Normalize(XfN12(dir, L.m2w));
@@ -756,7 +759,8 @@ DF V2 SquareToConcentricDisk(V2 u) {
         r = uOffset.y;
         theta = (kPI / 2) - (kPI / 4) * (uOffset.x / uOffset.y);
     }
-    float sinTheta = rt_sinf(theta), cosTheta = rt_cosf(theta);
+    float sinTheta, cosTheta;
+    rt_sincosf(theta, &sinTheta, &cosTheta);
     return v2(r * cosTheta, r * sinTheta);
 }
 /* LightEmitResult (Light.cs:61-107) without the unused uv */
@@ -784,7 +788,8 @@ NF Emit LightSampleEmit(const RtSceneView* S, int li, Rng& rand) {
             if (sinTheta != 0) {
                 pdf /= (2 * kPI * kPI * sinTheta);
                 float cosTheta = rt_cosf(theta);
-                float sinPhi = rt_sinf(phi), cosPhi = rt_cosf(phi);
+                float sinPhi, cosPhi;
+                rt_sincosf(phi, &sinPhi, &cosPhi);
                 V3 sph = v3(cosPhi * sinTheta, sinPhi * sinTheta, cosTheta);
                 V3 dir = v3(sph.y, sph.z, -sph.x);
                 worldDir = Normalize(XfN12(dir, L.m2w));
