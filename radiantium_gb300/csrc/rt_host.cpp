@@ -189,12 +189,12 @@ void free_wf(Ctx* c) {
     c->wf_slots = 0;
 }
 
-/* path-state arrays for `slots` paths in flight (about 560 bytes per slot: 1.1 GiB at 2 Mi slots) */
+/* path-state arrays for `slots` paths in flight (about 600 bytes per slot: 1.2 GiB at 2 Mi slots) */
 void ensure_wf(Ctx* c, int slots) {
     if (c->wf_slots >= slots) return;
     free_wf(c);
     WfState& W = c->wf;
-    const size_t n = (size_t)slots, q = 3 * (size_t)slots;
+    const size_t n = (size_t)slots, q = 4 * (size_t)slots;
     W.q_o = wf_alloc<float4>(c, q); W.q_d = wf_alloc<float4>(c, q); W.q_meta = wf_alloc<int32_t>(c, q);
     W.active[0] = wf_alloc<int32_t>(c, n); W.active[1] = wf_alloc<int32_t>(c, n);
     W.sorted = wf_alloc<int32_t>(c, n); W.sort_key = wf_alloc<uint16_t>(c, n); W.mark = wf_alloc<uint8_t>(c, n);
@@ -1046,6 +1046,7 @@ void particle_wavefront(Ctx* c, const RtParams& P, int64_t first, int64_t count,
     W.shadow_base = 2 * slots;
     W.refill = c->wf_refill;
     W.iter_cap = c->wf_iter_cap;
+    W.mis_any = c->counting ? 0 : 1;
     W.dense_sort = 1;
     WfMode m;
     m.particle = true;
@@ -1342,6 +1343,7 @@ void wavefront_run(Ctx* c, const std::vector<WfJobIn>& jobs, cudaStream_t s, boo
         W.shadow_base = 2 * slots;
         W.refill = c->wf_refill;
         W.iter_cap = c->wf_iter_cap;
+        W.mis_any = c->counting ? 0 : 1;
         /* vol_path's shade runs slower from slots walked in index order (C3: 115.3 -> 112.5 M samples/s) */
         W.dense_sort = mode.vol ? 0 : 1;
         /* one pass over the round's samples: start every slot, bounce until no path is left */

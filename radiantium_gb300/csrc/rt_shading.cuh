@@ -675,6 +675,23 @@ DF C3 EvalAllInfinite(const RtSceneView* S, V3 rd) {
     for (int i = 0; i < S->infinite_count; i++) l = l + InfLe(S, S->lights[S->infinite_lights[i]], rd);
     return l;
 }
+/* Light.PdfLi of infinite light `li` in direction wi (w), and where it is not
+ * 0 what Scene.EvalAllInfiniteLights gives there (xyz): the two look the same
+ * direction up in the same map */
+NF float4 EnvPdfLe(const RtSceneView* S, int li, V3 wi) {
+    const RtLight& L = S->lights[li];
+    V3 dir = Normalize(XfN12(wi, L.w2m));
+    float phi = rt_atan2f(dir.x, -dir.z);
+    phi = (phi < 0) ? (phi + 2 * kPI) : phi;
+    float theta = rt_acosf(nclamp(dir.y, -1, 1));
+    float sinTheta = rt_sinf(theta);
+    if (sinTheta == 0.0f) return make_float4(0, 0, 0, 0);
+    float u = phi / (2 * kPI), v = theta / kPI;
+    const float pdf = Pdf2D(S, S->dists[L.dist], u, v) / (2 * kPI * kPI * sinTheta);
+    C3 le = c3s(0.0f);
+    if (pdf != 0.0f) le = S->infinite_count == 1 ? c3s(0.0f) + TexSample(S, L.ref, v2(u, v)) : EvalAllInfinite(S, wi);
+    return make_float4(le.r, le.g, le.b, pdf);
+}
 /* Scene.SampleLight: uniform choice, pdf 1/N */
 DF float SampleLight(const RtSceneView* S, Rng& rand, int* light) {
     if (S->light_count == 0) { *light = -1; return 0.0f; }

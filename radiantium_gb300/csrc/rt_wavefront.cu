@@ -52,6 +52,7 @@ enum : uint32_t {
     F_WTR = 256u,        /* vol_path: a Transmittance-walk segment is being traced */
     F_WIT = 512u,        /* vol_path: an IntersectTr-walk segment is being traced */
     F_CONT = 1024u,      /* vol_path: the next extension ray waits for the pending term */
+    F_ANY = 4096u,       /* the pending BSDF-sample term's ray is an any-hit ray (WF_RAY_MIS_ANY) */
     F_ALL = 2048u,       /* path, All light strategy: the vertex's lights are estimated one per iteration */
 };
 
@@ -74,17 +75,17 @@ DF int warp_append(int* counter, bool want) {
 }
 
 /* Appends a shade's rays and its slot for the next iteration in one pass:
- * the shadow queue, the closest-hit queue (the warp's MIS rays, then its
- * extension rays) and the next active list `next`.  kBlock: one atomic per
+ * the any-hit queue (the warp's shadow rays, then its WF_RAY_MIS_ANY rays),
+ * the closest-hit queue (its MIS rays, then its extension rays) and the next active list `next`.  kBlock: one atomic per
  * counter per block, every thread of the block calls it (blockDim.x a
  * multiple of 32); else one per warp, every lane of the warp calls it.  The
  * three counters' atomics are in flight together.  Outputs are queue
  * positions (the shadow one including shadow_base), -1 where not wanted. */
 template <bool kBlock>
-DF void queue_append(const WfState& W, int next, bool shadow, bool mis, bool ext, bool keep,
-                     int* qs, int* qm, int* qe, int* qa) {
+DF void queue_append(const WfState& W, int next, bool shadow, bool any, bool mis, bool ext, bool keep,
+                     int* qs, int* qx, int* qm, int* qe, int* qa) {
     const unsigned full = 0xffffffffu;
-    const unsigned bs = __ballot_sync(full, shadow), bm = __ballot_sync(full, mis),
+    const unsigned bs = __ballot_sync(full, shadow), bx = __ballot_sync(full, any), bm = __ballot_sync(full, mis),
                    be = __ballot_sync(full, ext), ba = __ballot_sync(full, keep);
     const int lane = threadIdx.x & 31;
     int b0, b1, b2;
@@ -92,7 +93,7 @@ DF void queue_append(const WfState& W, int next, bool shadow, bool mis, bool ext
         __shared__ int s_cnt[3][32];
         __shared__ int s_base[3];
         const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        if (lane == 0) { s_cnt[0][w] = __popc(bs); s_cnt[1][w] = __popc(bm) + __popc(be); s_cnt[2][w] = __popc(ba); }
+        if (lane == 0) { s_cnt[0][w] = __popc(bs) + __popc(bx); s_cnt[1][w] = __popc(bm) + __popc(be); s_cnt[2][w] = __popc(ba); }
         __syncthreads();
         if (threadIdx.x < 3) {
             int* c = threadIdx.x == 0 ? &W.ctr->n_shadow : (threadIdx.x == 1 ? &W.ctr->n_closest : &W.ctr->n_active[next]);
@@ -106,7 +107,7 @@ DF void queue_append(const WfState& W, int next, bool shadow, bool mis, bool ext
     } else {
         int v = 0;
         if (lane < 3) {
-            const int t = lane == 0 ? __popc(bs) : (lane == 1 ? __popc(bm) + __popc(be) : __popc(ba));
+            const int t = lane == 0 ? __popc(bs) + __popc(bx) : (lane == 1 ? __popc(bm) + __popc(be) : __popc(ba));
             int* c = lane == 0 ? &W.ctr->n_shadow : (lane == 1 ? &W.ctr->n_closest : &W.ctr->n_active[next]);
             if (t) v = atomicAdd(c, t);
         }
@@ -114,6 +115,7 @@ DF void queue_append(const WfState& W, int next, bool shadow, bool mis, bool ext
     }
     const unsigned lt = (1u << lane) - 1u;
     *qs = shadow ? W.shadow_base + b0 + __popc(bs & lt) : -1;
+    *qx = any ? W.shadow_base + b0 + __popc(bs) + __popc(bx & lt) : -1;
     *qm = mis ? b1 + __popc(bm & lt) : -1;
     *qe = ext ? b1 + __popc(bm) + __popc(be & lt) : -1;
     *qa = keep ? b2 + __popc(ba & lt) : -1;
@@ -141,7 +143,7 @@ DF void clear_active(const WfState& W, int slot) {
 }
 
 DF void push_ray4(const WfState& W, int q, int path, int kind, float4 o, float4 d) {
-    if (!in_bounds(W, q, 3LL * W.slots)) return;
+    if (!in_bounds(W, q, 4LL * W.slots)) return;
     W.q_o[q] = o;
     W.q_d[q] = d;
     W.q_meta[q] = (path << 10) | ((int)W.job[path] << 2) | kind;
@@ -236,8 +238,8 @@ __global__ void __launch_bounds__(256) k_wf_start(WfState W) {
     const long long sid = claim_sample(W, 0xffffffffu, in);
     float4 o, d;
     const bool ok = in && init_path(W, slot, sid, &o, &d);
-    int qs, qm, qe, qa;
-    queue_append<true>(W, 0, false, false, ok, false, &qs, &qm, &qe, &qa);
+    int qs, qx, qm, qe, qa;
+    queue_append<true>(W, 0, false, false, false, ok, false, &qs, &qx, &qm, &qe, &qa);
     if (ok) push_ray4(W, qe, slot, WF_RAY_EXT, o, d);
 }
 
@@ -318,7 +320,9 @@ template <> struct TraceStack<true> {
  * way (the reference's `lock (renderTarget)` add, AdjointParticleIntegrator.cs:53-66) */
 DF void shadow_done(const WfState& W, int meta, bool hit) {
     const int path = meta_path(meta);
-    if (meta_kind(meta) != WF_RAY_SPLAT) { W.occluded[path] = hit ? 1 : 0; return; }
+    const int kind = meta_kind(meta);
+    if (kind == WF_RAY_SHADOW) { W.occluded[path] = hit ? 1 : 0; return; }
+    if (kind == WF_RAY_MIS_ANY) { W.mis_sub[path] = hit ? 1 : 0; return; }
     if (hit) return;
     const float4 sp = W.pd_l1[path];
     const int pix = __float_as_int(sp.w);
@@ -420,11 +424,11 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_CLOSEST_BLOCKS) k_wf_trace_
     trace_queue<false, kSh, kMode>(W, 0, min(W.ctr->n_closest, 2 * W.slots), &W.ctr->fetch[0], status, stats, counting);
 }
 
-/* shadow rays: any-hit (queue [shadow_base, shadow_base + n_shadow)) */
+/* shadow rays and infinite lights' MIS rays: any-hit (queue [shadow_base, shadow_base + n_shadow)) */
 template <bool kSh, NodeMode kMode>
 __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_SHADOW_BLOCKS) k_wf_trace_shadow(WfState W, uint32_t* status, unsigned long long* stats,
                                                            bool counting) {
-    trace_queue<true, kSh, kMode>(W, W.shadow_base, min(W.ctr->n_shadow, W.slots), &W.ctr->fetch[1], status, stats,
+    trace_queue<true, kSh, kMode>(W, W.shadow_base, min(W.ctr->n_shadow, 2 * W.slots), &W.ctr->fetch[1], status, stats,
                                   counting);
 }
 
@@ -479,13 +483,24 @@ DF void finish_path(const WfJob& J, const WfState& W, int slot, C3 rad, unsigned
 /* one bounce of PathTracer.Mis / NextEventEstimation / OnlySampleBxdf after the
  * extension hit is known (PathTracer.cs:43-270) */
 /* What a path shade leaves for the queues: its shadow ray, whether it
- * queued a MIS ray (in pd_ray_o / pd_ray_d) or an extension ray (in ray_o /
- * ray_d), whether the slot stays active, and whether the path is over (the
+ * queued a MIS ray (in pd_ray_o / pd_ray_d; mis_any: as an any-hit ray) or an
+ * extension ray (in ray_o / ray_d), whether the slot stays active, and whether the path is over (the
  * caller starts the next camera sample in the slot). */
 struct PathOut {
     float4 so, sd;
-    bool shadow, mis, ext, keep, restart;
+    bool shadow, mis_any, mis, ext, keep, restart;
 };
+
+/* The MIS ray towards an infinite light: EstimateDirect (PathTracer.cs:370-399)
+ * takes the radiance of what the ray hits only where that is the sampled light
+ * itself, which no primitive is, and the environment where it hits nothing.
+ * So the ray stops at its first hit - the same answer as the closest hit's
+ * existence - and the term it gates is complete when it is queued: the next
+ * shade adds it as it adds a light-sample term, without an intersection or the
+ * ray's direction and BSDF value.  A ray that could carry nothing is not traced. */
+DF bool MisAny(const WfState& W, const RtSceneView* S, int light) {
+    return W.mis_any && S->lights[light].kind == RT_LIGHT_INFINITE;
+}
 
 /* Schedules one light's direct term at vertex `it` (PathTracer.cs:309-399
  * for Mis, :95-190 for Nee): draws its light sample and, for Mis, its BSDF
@@ -526,26 +541,47 @@ DF void schedule_direct(PathOut* o, const WfState& W, const RtSceneView* S, int 
             float scatteringPdf = sample.Pdf;
             bool sampledSpecular = (sample.Type & BX_SPECULAR) != 0;
             if (!IsBlack(fr) && scatteringPdf > 0) {
+                const V3 wiw = Wo(it, sample.Wi);
+                const bool any = MisAny(W, S, light);
+                C3 env = c3s(0.0f);          /* any: the radiance the ray carries if it hits nothing */
                 float weight = 1;
                 bool go = true;
                 if (!sampledSpecular) {
-                    float bxdfToLightPdf = LightPdfLi(S, light, it.P, Wo(it, sample.Wi));
+                    float bxdfToLightPdf;
+                    if (any) {
+                        const float4 e = EnvPdfLe(S, light, wiw);
+                        env = c3(e.x, e.y, e.z);
+                        bxdfToLightPdf = e.w;
+                    } else {
+                        bxdfToLightPdf = LightPdfLi(S, light, it.P, wiw);
+                    }
                     if (bxdfToLightPdf == 0.0f) go = false;
                     else weight = PowerHeuristic(scatteringPdf, bxdfToLightPdf);
+                } else if (any) {
+                    env = EvalAllInfinite(S, wiw);
                 }
                 if (go) {
                     if (kAdj && __float_as_int(rho.w) >= 0)
                         rho.y = DirectDln(S, mat, Lo(it, wod), sample.Wi, sampledSpecular ? 2.0f : weight, false,
                                           it.UV);
-                    Ray toLight = Spawn(it, Wo(it, sample.Wi));
-                    V3 wle = Wo(it, -sample.Wi);
-                    W.pd_fr[slot] = make_float4(fr.r, fr.g, fr.b, weight);
-                    W.pd_mis[slot] = make_float4(scatteringPdf, __int_as_float(light), 0, 0);
-                    W.pd_w[slot] = make_float4(wle.x, wle.y, wle.z, 0);
-                    W.pd_ray_o[slot] = make_float4(toLight.O.x, toLight.O.y, toLight.O.z, toLight.MinT);
-                    W.pd_ray_d[slot] = make_float4(toLight.D.x, toLight.D.y, toLight.D.z, toLight.MaxT);
-                    fl |= F_L2;
-                    o->mis = true;
+                    const Ray toLight = Spawn(it, wiw);
+                    if (!any) {
+                        V3 wle = Wo(it, -sample.Wi);
+                        W.pd_fr[slot] = make_float4(fr.r, fr.g, fr.b, weight);
+                        W.pd_mis[slot] = make_float4(scatteringPdf, __int_as_float(light), 0, 0);
+                        W.pd_w[slot] = make_float4(wle.x, wle.y, wle.z, 0);
+                        fl |= F_L2;
+                        o->mis = true;
+                    } else if (!IsBlack(env)) {
+                        const C3 l2 = fr * env * weight / scatteringPdf;
+                        W.pd_fr[slot] = make_float4(l2.r, l2.g, l2.b, 0);
+                        fl |= F_L2 | F_ANY;
+                        o->mis_any = true;
+                    }
+                    if (o->mis || o->mis_any) {
+                        W.pd_ray_o[slot] = make_float4(toLight.O.x, toLight.O.y, toLight.O.z, toLight.MinT);
+                        W.pd_ray_d[slot] = make_float4(toLight.D.x, toLight.D.y, toLight.D.z, toLight.MaxT);
+                    }
                 }
             }
         } else {
@@ -613,7 +649,13 @@ DF void shade_path(PathOut* o, const WfState& W, int slot, uint32_t* status, uns
                     tl = c3(l1.x, l1.y, l1.z);
                     le = le + tl;
                 }
-                if (fl & F_L2) {
+                if ((fl & F_L2) && (fl & F_ANY)) {
+                    if (!W.mis_sub[slot]) {
+                        const float4 l2 = W.pd_fr[slot];
+                        tb = c3(l2.x, l2.y, l2.z);
+                        le = le + tb;
+                    }
+                } else if (fl & F_L2) {
                     float4 fr2 = W.pd_fr[slot];
                     float4 mi = W.pd_mis[slot];
                     float4 wl = W.pd_w[slot];
@@ -656,7 +698,7 @@ DF void shade_path(PathOut* o, const WfState& W, int slot, uint32_t* status, uns
             if (!(fl & F_DZERO) && !W.occluded[slot]) { float4 l1 = W.pd_l1[slot]; e = c3(l1.x, l1.y, l1.z); }
             radiance = all ? radiance + coeffb * e : radiance + coeffb * e / lightPdf;
         }
-        fl &= ~(F_PENDING | F_L1 | F_L2 | F_DZERO);
+        fl &= ~(F_PENDING | F_L1 | F_L2 | F_DZERO | F_ANY);
         if (all) {
             const float4 ac = W.pd_acc[slot];
             const int next = __float_as_int(ac.w) + 1;
@@ -799,9 +841,10 @@ DF void path_queues(const WfState& W, int slot, int next, PathOut& o) {
     const long long sid = claim_sample(W, 0xffffffffu, o.restart);
     float4 ro, rd;
     if (o.restart && init_path(W, slot, sid, &ro, &rd)) { o.ext = true; o.keep = true; }
-    int qs, qm, qe, qa;
-    queue_append<kBlock>(W, next, o.shadow, o.mis, o.ext, o.keep, &qs, &qm, &qe, &qa);
+    int qs, qx, qm, qe, qa;
+    queue_append<kBlock>(W, next, o.shadow, o.mis_any, o.mis, o.ext, o.keep, &qs, &qx, &qm, &qe, &qa);
     if (o.shadow) push_ray4(W, qs, slot, WF_RAY_SHADOW, o.so, o.sd);
+    if (o.mis_any) push_ray4(W, qx, slot, WF_RAY_MIS_ANY, W.pd_ray_o[slot], W.pd_ray_d[slot]);
     if (o.mis) push_ray4(W, qm, slot, WF_RAY_MIS, W.pd_ray_o[slot], W.pd_ray_d[slot]);
     if (o.ext) {
         if (!o.restart) { ro = W.ray_o[slot]; rd = W.ray_d[slot]; }
@@ -1169,8 +1212,8 @@ DF void vol_queues(const WfState& W, int slot, int next, VolOut& o) {
     const long long sid = claim_sample(W, 0xffffffffu, o.restart);
     float4 ro, rd;
     if (o.restart && init_path(W, slot, sid, &ro, &rd)) { o.ext = true; o.keep = true; }
-    int qs, qt, qe, qa;
-    queue_append<true>(W, next, false, o.trw, o.itw || o.ext, o.keep, &qs, &qt, &qe, &qa);
+    int qs, qx, qt, qe, qa;
+    queue_append<true>(W, next, false, false, o.trw, o.itw || o.ext, o.keep, &qs, &qx, &qt, &qe, &qa);
     if (o.trw) {
         float4 to, td;
         trw_ray(W, slot, &to, &td);
@@ -1221,7 +1264,7 @@ __global__ void __launch_bounds__(128, (kAdj || kDynamic) ? 5 : RT_SHADE_BLOCKS)
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
         int slot = -1;
         PathOut o;
-        o.shadow = o.mis = o.ext = o.keep = o.restart = false;
+        o.shadow = o.mis_any = o.mis = o.ext = o.keep = o.restart = false;
         if (i < n) { slot = list[i]; shade_path<kAdj>(&o, W, slot, status, stats, counting, pass, A, s_alpha); }
         path_queues<true>(W, slot, cur ^ 1, o);
     } else {
@@ -1234,7 +1277,7 @@ __global__ void __launch_bounds__(128, (kAdj || kDynamic) ? 5 : RT_SHADE_BLOCKS)
             const int i = base + lane;
             int slot = -1;
             PathOut o;
-            o.shadow = o.mis = o.ext = o.keep = o.restart = false;
+            o.shadow = o.mis_any = o.mis = o.ext = o.keep = o.restart = false;
             if (i < n) { slot = list[i]; shade_path<kAdj>(&o, W, slot, status, stats, counting, pass, A, s_alpha); }
             __syncwarp();
             path_queues<false>(W, slot, cur ^ 1, o);
@@ -1329,8 +1372,8 @@ DF long long claim_particle(const WfState& W, bool want) {
 
 /* queue the block's splat and extension rays and its next active slots */
 DF void particle_queues(const WfState& W, int slot, int next, const PartOut& o) {
-    int qs, qm, qe, a;
-    queue_append<true>(W, next, o.splat, false, o.ext, o.keep, &qs, &qm, &qe, &a);
+    int qs, qx, qm, qe, a;
+    queue_append<true>(W, next, o.splat, false, false, o.ext, o.keep, &qs, &qx, &qm, &qe, &a);
     if (o.splat) push_ray4(W, qs, slot, WF_RAY_SPLAT, o.so, o.sd);
     if (o.ext) push_ray4(W, qe, slot, WF_RAY_EXT, o.eo, o.ed);
     if (o.keep) set_active(W, next, a, slot);
@@ -1345,8 +1388,8 @@ __global__ void __launch_bounds__(256) k_wf_start_particles(WfState W) {
     const long long sid = claim_particle(W, in);
     if (in) start_particle(W, slot, sid, &o);
     /* the first active list is built from the slots' flags afterwards */
-    int qs, qm, qe, a;
-    queue_append<true>(W, 0, false, false, o.ext, false, &qs, &qm, &qe, &a);
+    int qs, qx, qm, qe, a;
+    queue_append<true>(W, 0, false, false, false, o.ext, false, &qs, &qx, &qm, &qe, &a);
     if (o.ext) push_ray4(W, qe, slot, WF_RAY_EXT, o.eo, o.ed);
 }
 

@@ -19,9 +19,11 @@
 /* ray kinds: extension, shadow (any hit), MIS / IntersectTr-walk segment,
  * Transmittance-walk segment (the last three closest hit except shadow).
  * In the shadow queue, WF_RAY_SPLAT marks a light-tracer camera connection:
- * the trace kernel adds its pending splat to the film when the way is clear. */
+ * the trace kernel adds its pending splat to the film when the way is clear;
+ * WF_RAY_MIS_ANY is the MIS ray of an infinite light, which counts only where
+ * it leaves the scene: whether it hits anything is all that is asked. */
 enum { WF_RAY_EXT = 0, WF_RAY_SHADOW = 1, WF_RAY_MIS = 2, WF_RAY_TRW = 3 };
-enum { WF_RAY_SPLAT = 2 };
+enum { WF_RAY_SPLAT = 2, WF_RAY_MIS_ANY = 3 };
 
 #define WF_MAX_JOBS 256            /* job index is 8 bits in the ray-queue meta word */
 #define WF_MAX_SLOTS (1 << 21)     /* slot index is 21 bits in the ray-queue meta word */
@@ -68,17 +70,18 @@ struct WfCounters {
 };
 
 /* structure-of-arrays path state; every array has one entry per path slot
- * except the ray queue (3 entries per slot) */
+ * except the ray queue (4 entries per slot) */
 struct WfState {
     /* ray queue: origin + MinT, direction + MaxT, (slot << 10) | (job << 2) | kind.
-     * Closest-hit rays (extension, MIS) fill [0, 2 * slots), shadow rays
-     * [shadow_base, shadow_base + slots): the two ray kinds never share a warp. */
+     * Closest-hit rays (extension, MIS) fill [0, 2 * slots), any-hit rays
+     * [shadow_base, shadow_base + 2 * slots): the two ray kinds never share a warp. */
     float4* q_o; float4* q_d; int32_t* q_meta;
     int32_t shadow_base;
     int32_t slots;
     uint32_t* status;        /* the context's status word (RT_STATUS_*) */
     int32_t refill;          /* idle lanes of a trace warp before it fetches new rays */
     int32_t iter_cap;        /* bounce iterations of one round before the run gives up (WF_ITER_CAP) */
+    int32_t mis_any;         /* infinite lights' MIS rays are any-hit rays (not while counting rays) */
     int32_t dense_sort;      /* the shade-key sort may walk the slots in index order (not for vol_path) */
     WfCounters* ctr;
     const WfJob* jobs;
@@ -99,14 +102,14 @@ struct WfState {
     float4* pd_coeff;        /* coeff at the bounce, light selection pdf */
     float4* pd_l1;           /* light-sample term (NEE: the whole estimate; light tracing:
                                 the splat's colour and film pixel) */
-    float4* pd_fr;           /* BSDF-sample f*cos, MIS weight */
+    float4* pd_fr;           /* BSDF-sample f*cos, MIS weight; any-hit MIS ray: its whole term */
     float4* pd_mis;          /* BSDF pdf, light index */
     float4* pd_w;            /* direction passed to the light's L() */
     float4* pd_ray_o; float4* pd_ray_d;
     float4* pd_acc;          /* All light strategy: the vertex's summed direct terms, light index (int bits) */
     /* ray results */
     float4* ext_hit; int32_t* ext_sub;
-    float4* mis_hit; int32_t* mis_sub;
+    float4* mis_hit; int32_t* mis_sub;   /* WF_RAY_MIS_ANY: mis_sub is 1 where the ray hit anything */
     uint8_t* occluded;
     /* adjoint replay: d ln (f w) / d alpha of the pending light and BSDF terms,
      * d ln f / d alpha of the continuation, alpha slot of the pending vertex */
