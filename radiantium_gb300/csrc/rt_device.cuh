@@ -676,7 +676,7 @@ DF int VisitWideNode(const float4* nodes, int node, const Ray& r, Stk stack, int
 /* Scene.Intersect over the two-level scene, in both forms: the closest hit
  * (Bvh.Intersect(ray, out inct), Accelerators/Bvh.cs:174-232, and
  * InstancedPrimitive.Intersect, Primitive.cs:169-188, with world
- * T = Distance(ray.O, p)) and, kAny, the first hit found (Bvh.cs:126-172,
+ * T = Distance(ray.O, p)) and, any-hit, the first hit found (Bvh.cs:126-172,
  * Primitive.cs:162-167).  Boxes, MaxT culls and primitive tests happen in
  * exactly the order of the recursive form; the recursion is unrolled into a
  * state machine of two kinds of step, so that a warp can run the lanes that
@@ -699,7 +699,8 @@ struct Traversal {
     Best best;
     float pt, pu, pv; int pslot; uint32_t pflags;     /* the prototype's own closest hit */
     int cur, sp, base, leafSlot, leafLeft, topSlot, topLeft, inst;
-    bool any, inProto, pany;     /* kAny: `any` is the answer */
+    bool any, inProto, pany;     /* any-hit form: `any` is the answer */
+    bool first;                  /* kEitherHit: stop at the first hit */
     uint32_t guard;
 };
 
@@ -748,9 +749,13 @@ DF bool DescendStep(Traversal& T, Stk stack, uint32_t* status, TravStats* st) {
     return false;
 }
 
+/* What a ray asks for; kEitherHit: T.first tells. */
+enum HitForm { kClosestHit, kAnyHit, kEitherHit };
+
 /* One primitive, or the end of a level (T.cur < 0); true when the traversal has finished. */
-template <bool kAny, class Stk, bool kWide = false>
+template <HitForm kForm, class Stk, bool kWide = false>
 DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status, TravStats* st) {
+    const bool stop = kForm == kAnyHit || (kForm == kEitherHit && T.first);
     const bool fresh = T.cur != RT_NO_NODE;
     if (fresh || T.leafLeft > 0) {
         const int slot = fresh ? ~T.cur : T.leafSlot;
@@ -766,7 +771,7 @@ DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status
         if (kind != RT_KIND_INSTANCE) {
             float t, u, v;
             if (!PrimHit(S, kind, ref, s0, s1, s2, T.r, &t, &u, &v)) {
-            } else if (kAny) {
+            } else if (stop) {
                 T.any = true;
                 return true;
             } else if (T.inProto) {
@@ -810,7 +815,7 @@ DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status
     if (!T.inProto) return true;
     /* leave the prototype: the instance's candidate in world space */
     T.inProto = false;
-    if (!kAny && T.pany) {
+    if (!stop && T.pany) {
         const RtInstance& I = S->instances[T.inst];
         const float4 s1 = __ldg(S->slots + 3 * (int64_t)T.pslot + 1);
         const uint32_t kr = __float_as_uint(s1.w);
@@ -849,7 +854,7 @@ DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status
 }
 
 /* The whole traversal of one ray by one thread. */
-template <bool kAny, bool kWide = false>
+template <HitForm kForm, bool kWide = false>
 DF void Traverse(const RtSceneView* S, const Ray& ray, Traversal& T, int2* stack, uint32_t* status, TravStats* st) {
     if (TraversalBegin<kWide>(S, ray, T, st)) return;
     const bool general = st || S->general_trees;
@@ -862,7 +867,7 @@ DF void Traverse(const RtSceneView* S, const Ray& ray, Traversal& T, int2* stack
                 DescendStep<int2*, kNodesShort>(T, stack, status, nullptr);
             }
         }
-        if (T.cur < 0 && LeafStep<kAny, int2*, kWide>(S, T, stack, status, st)) return;
+        if (T.cur < 0 && LeafStep<kForm, int2*, kWide>(S, T, stack, status, st)) return;
     }
 }
 
@@ -870,7 +875,7 @@ DF void Traverse(const RtSceneView* S, const Ray& ray, Traversal& T, int2* stack
 template <bool kWide = false>
 DF bool SceneClosest(const RtSceneView* S, Ray& ray, Best* best, int2* stack, uint32_t* status, TravStats* st) {
     Traversal T;
-    Traverse<false, kWide>(S, ray, T, stack, status, st);
+    Traverse<kClosestHit, kWide>(S, ray, T, stack, status, st);
     *best = T.best;
     ray.MaxT = T.inProto ? T.wMaxT : T.r.MaxT;
     return T.any;
@@ -879,7 +884,7 @@ DF bool SceneClosest(const RtSceneView* S, Ray& ray, Best* best, int2* stack, ui
 template <bool kWide = false>
 DF bool SceneAny(const RtSceneView* S, const Ray& ray, int2* stack, uint32_t* status, TravStats* st) {
     Traversal T;
-    Traverse<true, kWide>(S, ray, T, stack, status, st);
+    Traverse<kAnyHit, kWide>(S, ray, T, stack, status, st);
     return T.any;
 }
 

@@ -121,6 +121,7 @@ struct Ctx {
     WfJob* d_jobs = nullptr;                   /* device job table (WF_MAX_JOBS entries) */
     WfJob* h_jobs = nullptr;                   /* pinned staging of the job table */
     int wf_capacity = WF_MAX_SLOTS;            /* path slots in flight */
+    int wf_finish = -1;                        /* active paths from which one kernel ends a round; -1: finish_at's rule (test hook) */
     int wf_refill = RT_WF_REFILL;              /* idle lanes before a trace warp fetches (1..32) */
     bool wf_graph_pref = false;                /* RT_RENDERER_AUTO drives the wavefront as a graph */
     int gpu_build_min = 1 << 15;               /* trees of at least this many primitives build on the GPU */
@@ -964,6 +965,7 @@ struct WfMode {
     bool deep = false;       /* trace kernels with the shared-memory stack (trees of 16+ levels) */
     bool wide = false;       /* the opt-in fast traversal over the wide nodes */
     bool general = false;    /* a scene's trees need the general node visit */
+    bool one_type = false;   /* one scene, one material type */
 };
 /* CUDA-event times and launch counts of a run, summed over its rounds */
 struct WfTotals {
@@ -971,19 +973,55 @@ struct WfTotals {
     uint64_t launches = 0, trace_launches = 0;
 };
 
+/* Active paths from which rt_wf_finish ends a round (measured, ms; off / 8 Ki /
+ * 32 Ki / 64 Ki / 128 Ki paths): volume 26.9 / 21.5 / 20.7 / 20.6 / 21.5, light
+ * tracer 15.7 / 13.5 / 13.3 / 13.3 / 13.6, gradient step 5.26 / 5.09 / 5.06 / 5.02
+ * / 5.02.  Its warps take the paths unsorted, so scenes of several material
+ * types gain less and lose it sooner: batch of twelve 35.5 / 34.8 / 35.0 / 35.1 /
+ * 36.1, zoo with all lights 11.6 / 11.6 / 13.6 / 15.9 / 15.9. */
+int finish_at(const Ctx* c, const WfMode& m) {
+    if (c->wf_finish >= 0) return c->wf_finish;
+    return m.vol || m.particle || m.one_type ? 65536 : 8192;
+}
+
 /* One round of a wavefront run over the jobs already in c->d_jobs: every slot
- * takes a sample (or particle), then the loop bounces until no path is active
- * and no splat ray is queued (a finished particle leaves its last one behind).
+ * takes a sample (or particle), then the loop bounces until at most
+ * W.finish_max paths are active, which one more launch runs to their end
+ * (rt_wf_finish; with finish_max 0 the loop itself runs until no path is active
+ * and no splat ray is queued - a finished particle leaves its last one behind).
  * The loop runs as one CUDA graph launch (render passes with `use_graph`) or
- * is driven from the host with per-phase event timing. */
-void wf_round(Ctx* c, const WfState& W, cudaStream_t s, bool use_graph, const WfMode& m, int pass,
+ * is driven from the host with per-phase event timing; a round that starts
+ * with no more paths than finish_max has no loop. */
+void wf_round(Ctx* c, WfState W, cudaStream_t s, bool use_graph, const WfMode& m, int pass,
               const WfAdjoint* adj, int64_t total, int n_jobs, WfTotals* t) {
+    W.finish_max = pass == WF_PASS_REPLAY || c->counting || m.general ? 0 : finish_at(c, m);
     std::memset(c->h_ctr, 0, sizeof(WfCounters));
     c->h_ctr->total = total;
     c->h_ctr->n_jobs = n_jobs;
     h2d(c, c->d_ctr, c->h_ctr, sizeof(WfCounters), s);
     CK(rt_wf_start(W, s, m.particle));
     t->launches += 2;
+    auto add_ms = [&](int from, double* sum) {
+        float ms = 0;
+        CK(cudaEventElapsedTime(&ms, c->events[from], c->events[from + 1]));
+        *sum += ms;
+    };
+    /* the rays of the paths that are left, then the paths to their end; stream order, no wait */
+    auto end_round = [&]() {
+        CK(cudaEventRecord(c->events[0], s));
+        CK(rt_wf_trace(W, c->status, c->stats, c->counting, s, m.deep, m.wide, m.general, &c->fork));
+        CK(rt_wf_finish(W, c->status, c->stats, s, pass, m.vol, m.particle, m.wide));
+        CK(cudaEventRecord(c->events[1], s));
+        t->launches += 4;
+        t->trace_launches += 2;
+    };
+    if (W.finish_max > 0 && std::min<int64_t>(W.slots, total) <= W.finish_max) {
+        if (c->cancel.load()) throw RtFail(RT_ERR_CANCELLED, "render cancelled");
+        end_round();
+        CK(cudaStreamSynchronize(s));
+        add_ms(0, &t->trace_ms);
+        return;
+    }
     if (use_graph && pass == WF_PASS_RENDER) {
         ensure_wf_graph(c, W, m);
         CK(cudaEventRecord(c->events[0], s));
@@ -992,16 +1030,15 @@ void wf_round(Ctx* c, const WfState& W, cudaStream_t s, bool use_graph, const Wf
         CK(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(WfCounters), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         const uint64_t iters = (uint64_t)std::max(0, c->h_ctr->iter);
-        t->launches += (m.sort ? 7 : 5) * iters;
-        t->trace_launches += 2 * iters;
-        float ms = 0;
-        CK(cudaEventElapsedTime(&ms, c->events[0], c->events[1]));
-        t->trace_ms += ms;                     /* the whole loop: not split by phase */
+        t->launches += (m.sort ? 7 : 5) * iters + (W.finish_max > 0 ? 4 : 0);
+        t->trace_launches += 2 * iters + (W.finish_max > 0 ? 2 : 0);
+        add_ms(0, &t->trace_ms);               /* the whole loop: not split by phase */
         return;
     }
     CK(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(WfCounters), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    while (c->h_ctr->n_active[c->h_ctr->iter & 1] > 0 || c->h_ctr->n_shadow > 0) {
+    auto active = [&]() { return c->h_ctr->n_active[c->h_ctr->iter & 1]; };
+    while (active() > W.finish_max || (W.finish_max == 0 && c->h_ctr->n_shadow > 0)) {
         if (c->cancel.load()) throw RtFail(RT_ERR_CANCELLED, "render cancelled");
         if (c->h_ctr->iter >= W.iter_cap) throw RtFail(RT_ERR_ITER_CAP, "wavefront: bounce iteration cap reached (WF_ITER_CAP)");
         NvtxRange nvtx_iter("rt.wavefront_iteration");
@@ -1009,16 +1046,20 @@ void wf_round(Ctx* c, const WfState& W, cudaStream_t s, bool use_graph, const Wf
         CK(rt_wf_trace(W, c->status, c->stats, c->counting, s, m.deep, m.wide, m.general, &c->fork));
         CK(cudaEventRecord(c->events[1], s));
         CK(cudaEventRecord(c->events[2], s));
-        CK(rt_wf_shade(W, c->h_ctr->n_active[c->h_ctr->iter & 1], c->status, c->stats, c->counting, 0, false, s,
-                       &t->launches, pass, adj, m.vol, m.particle, m.sort));
+        CK(rt_wf_shade(W, active(), c->status, c->stats, c->counting, 0, false, s, &t->launches, pass, adj, m.vol,
+                       m.particle, m.sort));
         CK(cudaEventRecord(c->events[3], s));
         t->launches += 2;
         t->trace_launches += 2;
         CK(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(WfCounters), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        float ms = 0;
-        CK(cudaEventElapsedTime(&ms, c->events[0], c->events[1])); t->trace_ms += ms;
-        CK(cudaEventElapsedTime(&ms, c->events[2], c->events[3])); t->shade_ms += ms;
+        add_ms(0, &t->trace_ms);
+        add_ms(2, &t->shade_ms);
+    }
+    if (active() > 0 || c->h_ctr->n_shadow > 0) {
+        end_round();
+        CK(cudaStreamSynchronize(s));
+        add_ms(0, &t->trace_ms);
     }
 }
 
@@ -1247,7 +1288,7 @@ struct WfJobIn {
  * counting mode changes. */
 void ensure_wf_graph(Ctx* c, const WfState& W, const WfMode& m) {
     const uint64_t key = (c->wf_generation << 32) ^ ((uint64_t)m.wide << 63) ^ ((uint64_t)m.general << 62) ^ ((uint64_t)W.slots << 10) ^ ((uint64_t)m.deep << 9) ^
-                         ((uint64_t)(uint32_t)W.iter_cap * 0x9E3779B97F4A7C15ull) ^
+                         ((uint64_t)(uint32_t)W.iter_cap * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)(uint32_t)W.finish_max * 0xC2B2AE3D27D4EB4Full) ^
                          ((uint64_t)m.sort << 8) ^ ((uint64_t)m.particle << 7) ^ ((uint64_t)W.refill << 2) ^
                          ((uint64_t)m.vol << 1) ^ (c->counting ? 1u : 0u);
     if (c->wf_exec && c->wf_graph_key == key) return;
@@ -1273,6 +1314,14 @@ void ensure_wf_graph(Ctx* c, const WfState& W, const WfMode& m) {
     CK(cudaStreamEndCapture(c->stream, &captured));
     CK(e1);
     CK(e2);
+    if (W.finish_max > 0) {                    /* after the loop: the paths that are left */
+        CK(cudaStreamBeginCaptureToGraph(c->stream, c->wf_graph, &node, nullptr, 1, cudaStreamCaptureModeRelaxed));
+        e1 = rt_wf_trace(W, c->status, c->stats, c->counting, c->stream, m.deep, m.wide, m.general, &c->fork);
+        e2 = rt_wf_finish(W, c->status, c->stats, c->stream, WF_PASS_RENDER, m.vol, m.particle, m.wide);
+        CK(cudaStreamEndCapture(c->stream, &captured));
+        CK(e1);
+        CK(e2);
+    }
     CK(cudaGraphInstantiate(&c->wf_exec, c->wf_graph, 0));
     c->wf_graph_key = key;
 }
@@ -1298,7 +1347,8 @@ void wavefront_run(Ctx* c, const std::vector<WfJobIn>& jobs, cudaStream_t s, boo
      * gradients/s unsorted, 28.5 sorted), so both keep it. */
     WfMode mode;
     mode.vol = vol;
-    mode.sort = vol || adj || jobs.size() > 1 || jobs[0].mat_types > 1;
+    mode.one_type = jobs.size() == 1 && jobs[0].mat_types <= 1;
+    mode.sort = vol || adj || !mode.one_type;
     for (const WfJobIn& J : jobs) mode.deep = mode.deep || J.tallest >= RT_DEEP_TREE;
     mode.wide = c->traversal == RT_TRAVERSAL_WIDE;
     for (const WfJobIn& J : jobs) mode.wide = mode.wide && J.wide_ok;
@@ -1957,6 +2007,14 @@ int rt_debug_set_iter_cap(void* ctx, int cap) {
     Ctx* c = (Ctx*)ctx;
     if (!c || cap < 0) return RT_ERR_INVALID_ARG;
     c->wf_iter_cap = cap == 0 ? WF_ITER_CAP : cap;
+    return RT_OK;
+}
+/* test hook (not part of radiantium.h): active paths from which one kernel
+ * ends a wavefront round; 0: the loop runs to its end, -1: the built-in rule */
+int rt_debug_set_finish(void* ctx, int paths) {
+    Ctx* c = (Ctx*)ctx;
+    if (!c || paths < -1) return RT_ERR_INVALID_ARG;
+    c->wf_finish = paths;
     return RT_OK;
 }
 /* test hook: primitive count from which upload_scene builds trees on the GPU */

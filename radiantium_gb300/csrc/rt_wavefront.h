@@ -81,6 +81,7 @@ struct WfState {
     uint32_t* status;        /* the context's status word (RT_STATUS_*) */
     int32_t refill;          /* idle lanes of a trace warp before it fetches new rays */
     int32_t iter_cap;        /* bounce iterations of one round before the run gives up (WF_ITER_CAP) */
+    int32_t finish_max;      /* active slots from which rt_wf_finish ends the round; 0: the loop runs to its end */
     int32_t mis_any;         /* infinite lights' MIS rays are any-hit rays (not while counting rays) */
     int32_t dense_sort;      /* the shade-key sort may walk the slots in index order (not for vol_path) */
     WfCounters* ctr;
@@ -158,5 +159,12 @@ cudaError_t rt_wf_shade(const WfState& W, int n_hint, uint32_t* status, unsigned
                         cudaGraphConditionalHandle loop, bool has_loop, cudaStream_t s, uint64_t* launches,
                         int pass = WF_PASS_RENDER, const WfAdjoint* adj = nullptr, bool vol = false,
                         bool particle = false, bool sort = true);
+/* resets the queue counters between the trace and the shade of an iteration */
+cudaError_t rt_wf_phase(const WfState& W, cudaStream_t s);
+/* Ends the round in one launch (and rt_wf_phase): runs every active slot's
+ * path, whose rays have been traced, to its end (rt_finish.cu).  Not for the
+ * adjoint's replay, for counting or for scenes with general_trees. */
+cudaError_t rt_wf_finish(const WfState& W, uint32_t* status, unsigned long long* stats, cudaStream_t s, int pass,
+                         bool vol, bool particle, bool wide);
 
 #endif
