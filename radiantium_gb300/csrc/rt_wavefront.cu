@@ -56,17 +56,17 @@ __global__ void __launch_bounds__(256) k_wf_start(WfState W) {
 #define RT_SHADOW_BLOCKS 7
 #endif
 /* the same for the shade kernels of `path` (the host-driven render pass; the
- * graph-driven and adjoint-replay variants keep 5, where 6 spills far more)
- * and of the light tracer.  Path shade, M samples/s C2 / C1 / C4: 157.2 /
- * 444.3 / 443.2 at 6, 158.8 / 445.6 / 443.4 at 7; at 8, C2 159.9 but C1 440.1. */
+ * graph-driven and adjoint-replay variants keep 5, where 6 spills far more), of
+ * the light tracer and of vol_path.  Path shade at 6 / 7 / 8, ms: Cornell frame
+ * 7.54 / 7.33 / 7.42, instances 69.6 / 68.8 / 68.3, batch 34.1 / 33.5 / 33.8. */
 #ifndef RT_SHADE_BLOCKS
 #define RT_SHADE_BLOCKS 7
 #endif
 #ifndef RT_PSHADE_BLOCKS
-#define RT_PSHADE_BLOCKS 6
+#define RT_PSHADE_BLOCKS 7       /* light tracer, ms: 13.4 at 5, 13.2 at 6, 13.1 at 7 */
 #endif
 #ifndef RT_VSHADE_BLOCKS
-#define RT_VSHADE_BLOCKS 5       /* C3 M samples/s: 124.7 at 4, 126.1 at 5, 126.0 at 6 */
+#define RT_VSHADE_BLOCKS 6       /* volume, ms: 20.7 at 4, 20.4 at 5, 20.3 at 6 */
 #endif
 
 /* closest-hit rays: extension and MIS rays (queue [0, n_closest)) */

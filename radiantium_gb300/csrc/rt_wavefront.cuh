@@ -437,7 +437,7 @@ DF bool MisAny(const WfState& W, const RtSceneView* S, int light) {
  * or 1 (All). */
 template <bool kAdj>
 DF void schedule_direct(PathOut* o, const WfState& W, const RtSceneView* S, int slot, const Isect& it, V3 wo, int mat,
-                        int light, float lightPdf, C3 coeff, int method, Rng& rand, uint32_t& fl, float4& rho) {
+                        const MatAt& at, int light, float lightPdf, C3 coeff, int method, Rng& rand, uint32_t& fl, float4& rho) {
     if (method == RT_METHOD_MIS) {
         fl |= F_PENDING;
         W.pd_coeff[slot] = make_float4(coeff.r, coeff.g, coeff.b, lightPdf);
@@ -445,8 +445,9 @@ DF void schedule_direct(PathOut* o, const WfState& W, const RtSceneView* S, int 
             V3 wod = it.Wr;
             LSample ls = LightSampleLi(S, light, it.P, rand);
             if (ls.Pdf > 0.0f && !IsBlack(ls.Li)) {
-                C3 fr = MatFr(S, mat, Lo(it, wod), Lo(it, ls.Wi), it.UV);
-                float scatteringPdf = MatPdf(S, mat, Lo(it, wod), Lo(it, ls.Wi), it.UV);
+                const float4 ev = MatEval(S, mat, at, Lo(it, wod), Lo(it, ls.Wi));
+                C3 fr = c3(ev.x, ev.y, ev.z);
+                const float scatteringPdf = ev.w;
                 if (!IsBlack(fr)) {
                     /* IsOccluded(it.P, ls.P) */
                     V3 vec = ls.P - it.P;
@@ -464,7 +465,7 @@ DF void schedule_direct(PathOut* o, const WfState& W, const RtSceneView* S, int 
                     }
                 }
             }
-            BSample sample = MatSample(S, mat, Lo(it, wod), it.UV, rand);
+            BSample sample = MatSampleAt(S, mat, at, Lo(it, wod), rand);
             C3 fr = sample.Fr * AbsCosTheta(sample.Wi);
             float scatteringPdf = sample.Pdf;
             bool sampledSpecular = (sample.Type & BX_SPECULAR) != 0;
@@ -525,7 +526,7 @@ DF void schedule_direct(PathOut* o, const WfState& W, const RtSceneView* S, int 
                 V3 vec = r.P - it.P;
                 float dis = Length(vec);
                 if (!(dis < 0.001f)) {
-                    C3 fr = MatFr(S, mat, Lo(it, wo), Lo(it, r.Wi), it.UV);
+                    C3 fr = MatFrAt(S, mat, at, Lo(it, wo), Lo(it, r.Wi));
                     C3 e = fr * r.Li * AbsCosTheta(Lo(it, r.Wi)) / r.Pdf;
                     W.pd_l1[slot] = make_float4(e.r, e.g, e.b, 0);
                     zero = false;
@@ -640,8 +641,9 @@ DF void shade_path(PathOut* o, const WfState& W, int slot, uint32_t* status, uns
                 Rng rand;
                 rng_resume(rand, P.seed, (uint32_t)(P.x0 + px.x), (uint32_t)(P.y0 + px.y), (uint32_t)px.w, W.rng_n[slot]);
                 float4 rho = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
-                schedule_direct<kAdj>(o, W, S, slot, it, -ray.D, PrimOf(S, it).material, next, 1.0f, coeffb, P.method,
-                                      rand, fl, rho);
+                const int mat = PrimOf(S, it).material;
+                schedule_direct<kAdj>(o, W, S, slot, it, -ray.D, mat, MatLookup(S, S->materials[mat], it.UV), next, 1.0f,
+                                      coeffb, P.method, rand, fl, rho);
                 W.pd_acc[slot] = make_float4(ac.x, ac.y, ac.z, __int_as_float(next));
                 W.rng_n[slot] = rand.n;
                 W.flags[slot] = fl;
@@ -688,8 +690,12 @@ DF void shade_path(PathOut* o, const WfState& W, int slot, uint32_t* status, uns
                 if (!isHit) { done = true; break; }
                 if (P.max_depth != -1 && bounces >= P.max_depth) { done = true; break; }
                 if (!HasSurface(S, it)) { nray = mkray(it.P, ray.D, ray.MinT); ext = true; break; }
+            }
+            /* the vertex's texture values, for its direct light and its continuation */
+            const int mat = PrimOf(S, it).material;
+            const MatAt at = MatLookup(S, S->materials[mat], it.UV);
+            if (!resume && P.method != RT_METHOD_BXDF) {
                 /* direct lighting: everything but the two ray casts */
-                const int mat = PrimOf(S, it).material;
                 float4 rho = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
                 if (kAdj && grad) {
                     if (UsesAlbedo(S, A.albedo_tex, mat)) {
@@ -706,24 +712,24 @@ DF void shade_path(PathOut* o, const WfState& W, int slot, uint32_t* status, uns
                         /* light 0 now, the others one per iteration; the continuation waits */
                         fl |= F_ALL;
                         W.pd_acc[slot] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
-                        schedule_direct<kAdj>(o, W, S, slot, it, wo, mat, 0, 1.0f, coeff, P.method, rand, fl, rho);
+                        schedule_direct<kAdj>(o, W, S, slot, it, wo, mat, at, 0, 1.0f, coeff, P.method, rand, fl, rho);
                         break;
                     }
                     if (P.method == RT_METHOD_MIS) radiance = radiance + coeff * c3s(0.0f);
                 } else {
                     int light;
                     float lightPdf = SampleLight(S, rand, &light);
-                    schedule_direct<kAdj>(o, W, S, slot, it, wo, mat, light, lightPdf, coeff, P.method, rand, fl, rho);
+                    schedule_direct<kAdj>(o, W, S, slot, it, wo, mat, at, light, lightPdf, coeff, P.method, rand, fl, rho);
                 }
                 if (kAdj) W.adj_rho[slot] = rho;
             }
             /* continuation */
-            BSample s = MatSample(S, PrimOf(S, it).material, Lo(it, wo), it.UV, rand);
+            BSample s = MatSampleAt(S, mat, at, Lo(it, wo), rand);
             if (kAdj && P.method == RT_METHOD_MIS && (fl & F_PENDING)) {
                 float4 rho = W.adj_rho[slot];
                 float rc = 0.0f, rcp;
                 if (__float_as_int(rho.w) >= 0 && s.Pdf > 0.0f)
-                    DlnAlpha(S, PrimOf(S, it).material, Lo(it, wo), s.Wi, it.UV, &rc, &rcp);
+                    DlnAlpha(S, mat, Lo(it, wo), s.Wi, it.UV, &rc, &rcp);
                 rho.z = rc;
                 W.adj_rho[slot] = rho;
             }
@@ -1032,6 +1038,7 @@ DF void shade_vol_path(VolOut* o, const WfState& W, int slot, uint32_t* status, 
                     break;
                 }
                 const int mat = PrimOf(S, it).material;
+                const MatAt at = MatLookup(S, S->materials[mat], it.UV);
                 int light;
                 const float lightPdf = SampleLight(S, rand, &light);
                 fl |= F_PENDING;
@@ -1040,8 +1047,9 @@ DF void shade_vol_path(VolOut* o, const WfState& W, int slot, uint32_t* status, 
                     const V3 wod = it.Wr;
                     const LSample ls = LightSampleLi(S, light, it.P, rand);
                     if (ls.Pdf > 0.0f && !IsBlack(ls.Li)) {
-                        C3 fr = MatFr(S, mat, Lo(it, wod), Lo(it, ls.Wi), it.UV);
-                        const float scatteringPdf = MatPdf(S, mat, Lo(it, wod), Lo(it, ls.Wi), it.UV);
+                        const float4 ev = MatEval(S, mat, at, Lo(it, wod), Lo(it, ls.Wi));
+                        C3 fr = c3(ev.x, ev.y, ev.z);
+                        const float scatteringPdf = ev.w;
                         if (!IsBlack(fr)) {
                             fl |= F_L1 | F_WTR;
                             fr = fr * AbsCosTheta(Lo(it, ls.Wi));
@@ -1055,7 +1063,7 @@ DF void shade_vol_path(VolOut* o, const WfState& W, int slot, uint32_t* status, 
                             W.trw_tr[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
                         }
                     }
-                    const BSample sample = MatSample(S, mat, Lo(it, wod), it.UV, rand);
+                    const BSample sample = MatSampleAt(S, mat, at, Lo(it, wod), rand);
                     const C3 fr = sample.Fr * AbsCosTheta(sample.Wi);
                     const float scatteringPdf = sample.Pdf;
                     const bool sampledSpecular = (sample.Type & BX_SPECULAR) != 0;
@@ -1084,7 +1092,7 @@ DF void shade_vol_path(VolOut* o, const WfState& W, int slot, uint32_t* status, 
                 } else {
                     fl |= F_DZERO;
                 }
-                const BSample sample = MatSample(S, mat, Lo(it, wo), it.UV, rand);
+                const BSample sample = MatSampleAt(S, mat, at, Lo(it, wo), rand);
                 isSpecularPath = (sample.Type & BX_SPECULAR) != 0;
                 if (sample.Pdf > 0.0f) coeff = coeff * (sample.Fr * AbsCosTheta(sample.Wi) / sample.Pdf);
                 else { done = true; break; }
