@@ -20,11 +20,14 @@ namespace {
 
 enum FinishKind { kFinishPath, kFinishVol, kFinishParticle };
 
-/* resident blocks per SM (volume / light tracer / Cornell frame, ms: 20.6 / 13.3 / 7.78 at 4,
- * 20.5 / 13.0 / 7.53 at 3, 20.6 / 13.3 / 7.59 at 2): the shade and the traversal share a kernel,
- * and at 4 blocks' registers both spill */
+/* resident blocks per SM.  Path: a whole round of 64 Ki Cornell samples takes 0.39
+ * ms at 4 and 0.48 at 3 (more warps); vol_path and the light tracer, which take
+ * over long tails: 20.5 / 13.4 ms at 4, 20.4 / 13.3 at 3, 20.6 / 13.3 at 2. */
 #ifndef RT_FINISH_BLOCKS
 #define RT_FINISH_BLOCKS 3
+#endif
+#ifndef RT_FINISH_PATH_BLOCKS
+#define RT_FINISH_PATH_BLOCKS 4
 #endif
 #define RT_FINISH_MIN 4          /* fewest paths a warp takes at a time (1: the same) */
 #define RT_FINISH_REFILL 4       /* idle lanes before a warp hands out more of its rays (1: the same) */
@@ -33,7 +36,7 @@ enum FinishKind { kFinishPath, kFinishVol, kFinishParticle };
 /* Entered with the rays of the current active list traced (rt_wf_trace) and
  * the counters reset (rt_wf_phase). */
 template <FinishKind kKind, NodeMode kMode>
-__global__ void __launch_bounds__(WF_FINISH_BLOCK, RT_FINISH_BLOCKS) k_wf_finish(WfState W, uint32_t* status, unsigned long long* stats,
+__global__ void __launch_bounds__(WF_FINISH_BLOCK, kKind == kFinishPath ? RT_FINISH_PATH_BLOCKS : RT_FINISH_BLOCKS) k_wf_finish(WfState W, uint32_t* status, unsigned long long* stats,
                                                                 int pass) {
     __shared__ int s_rays[WF_FINISH_BLOCK / 32][3 * 32];
     int* const rays = s_rays[threadIdx.x >> 5];

@@ -975,13 +975,19 @@ struct WfTotals {
 
 /* Active paths from which rt_wf_finish ends a round (measured, ms; off / 8 Ki /
  * 32 Ki / 64 Ki / 128 Ki paths): volume 26.9 / 21.5 / 20.7 / 20.6 / 21.5, light
- * tracer 15.7 / 13.5 / 13.3 / 13.3 / 13.6, gradient step 5.26 / 5.09 / 5.06 / 5.02
- * / 5.02.  Its warps take the paths unsorted, so scenes of several material
- * types gain less and lose it sooner: batch of twelve 35.5 / 34.8 / 35.0 / 35.1 /
- * 36.1, zoo with all lights 11.6 / 11.6 / 13.6 / 15.9 / 15.9. */
+ * tracer 15.7 / 13.5 / 13.3 / 13.3 / 13.6.  Path tails are short (Cornell frame
+ * 7.68 / 7.67 / 7.78 / 7.78 / 7.79), and its warps take the paths unsorted, so
+ * scenes of several material types lose soonest: batch of twelve 35.5 / 34.8 /
+ * 35.0 / 35.1 / 36.1, zoo with all lights 11.6 / 11.6 / 13.6 / 15.9 / 15.9. */
 int finish_at(const Ctx* c, const WfMode& m) {
     if (c->wf_finish >= 0) return c->wf_finish;
-    return m.vol || m.particle || m.one_type ? 65536 : 8192;
+    return m.vol || m.particle ? 65536 : 8192;
+}
+/* Paths up to which a round has no loop at all, where the loop would make a
+ * handful of iterations of a few launches and a wait each: one material type,
+ * 64 Ki Cornell samples 0.52 ms with the loop and 0.39 without. */
+int whole_round(const Ctx* c, const WfMode& m) {
+    return m.one_type && c->wf_finish < 0 ? 65536 : finish_at(c, m);
 }
 
 /* One round of a wavefront run over the jobs already in c->d_jobs: every slot
@@ -1015,7 +1021,7 @@ void wf_round(Ctx* c, WfState W, cudaStream_t s, bool use_graph, const WfMode& m
         t->launches += 4;
         t->trace_launches += 2;
     };
-    if (W.finish_max > 0 && std::min<int64_t>(W.slots, total) <= W.finish_max) {
+    if (W.finish_max > 0 && std::min<int64_t>(W.slots, total) <= whole_round(c, m)) {
         if (c->cancel.load()) throw RtFail(RT_ERR_CANCELLED, "render cancelled");
         end_round();
         CK(cudaStreamSynchronize(s));
