@@ -6,6 +6,7 @@
 #include "rt_bvh.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <future>
@@ -90,7 +91,7 @@ public:
 
     /* appends the subtree of items [lo, hi) to `out` in depth-first order;
      * right-child indices are relative to the start of `out` */
-    int build(std::vector<FlatNode>& out, int lo, int hi, int level) {
+    int build(Array<FlatNode>& out, int lo, int hi, int level) {
         Box bounds = empty_box();
         for (int i = lo; i < hi; i++) box_union(bounds, items_[i].b);
         const int n = hi - lo;
@@ -144,7 +145,7 @@ public:
         out.push_back(node);
         int dl, dr;
         if (level < par_depth_ && n > 65536) {
-            std::vector<FlatNode> left, right;
+            Array<FlatNode> left, right;
             auto fut = std::async(std::launch::async, [&]() { return build(left, lo, mid, level + 1); });
             dr = build(right, mid, hi, level + 1);
             dl = fut.get();
@@ -163,13 +164,13 @@ public:
     }
 
 private:
-    static void splice(std::vector<FlatNode>& out, std::vector<FlatNode>& s) {
+    static void splice(Array<FlatNode>& out, Array<FlatNode>& s) {
         const int base = (int)out.size();
         for (FlatNode& n : s) {
             if (n.count == 0) n.second += base;
             out.push_back(n);
         }
-        std::vector<FlatNode>().swap(s);
+        Array<FlatNode>().swap(s);
     }
     std::vector<Item>& items_;
     int max_prims_;
@@ -178,7 +179,7 @@ private:
 
 }  // namespace
 
-BuildResult build_sah(const std::vector<Box>& prim_bounds, int max_prims, int threads) {
+BuildResult build_sah(const Array<Box>& prim_bounds, int max_prims, int threads) {
     BuildResult r;
     const int n = (int)prim_bounds.size();
     if (n == 0) return r;
@@ -200,34 +201,52 @@ BuildResult build_sah(const std::vector<Box>& prim_bounds, int max_prims, int th
 
 /* ---- the wide tree of the fast traversal -------------------------------------------------- */
 
+/* floor and ceil of log2(x), x > 0, and 2^k (-1022 <= k <= 1023) */
+static int floor_log2(double x) {
+    int e;
+    std::frexp(x, &e);
+    return e - 1;
+}
+static int ceil_log2(double x) {
+    int e;
+    const double m = std::frexp(x, &e);
+    return m == 0.5 ? e - 1 : e;
+}
+static double pow2(int k) {
+    const uint64_t bits = (uint64_t)(k + 1023) << 52;
+    double d;
+    std::memcpy(&d, &bits, 8);
+    return d;
+}
+
 /* The quantisation grid of one axis of a node box [mn, mx]: scale 2^k with k
  * large enough that 253 steps cover the extent and that one step is at least
  * 2^-20 of the coordinates' magnitude (so the one-step padding outweighs the
  * rounding of the traversal's plane distances), origin one step below mn
  * (rounded down).  Children are quantised outwards with one more step of
  * padding; k grows until every child fits in [0, 255]. */
-static void quantise_axis(double mn, double mx, const std::vector<std::pair<double, double>>& kids, float* p,
-                          uint8_t* e, uint8_t* qlo, uint8_t* qhi) {
+static void quantise_axis(double mn, double mx, const Box* kids, int n, int axis, float* p, uint8_t* e, uint8_t* qlo,
+                          uint8_t* qhi) {
     const double ext = mx - mn;
     const double mag = std::max(std::max(std::fabs(mn), std::fabs(mx)), 1e-30);
-    int k = std::max(ext > 0 ? (int)std::ceil(std::log2(ext / 253.0)) : -126, (int)std::floor(std::log2(mag)) - 20);
+    int k = std::max(ext > 0 ? ceil_log2(ext / 253.0) : -126, floor_log2(mag) - 20);
     for (k = std::max(k, -126); k <= 127; k++) {
-        const double s = std::ldexp(1.0, k);
+        const double s = pow2(k);
         float pf = (float)(mn - s);
         if ((double)pf > mn - s) pf = std::nextafter(pf, -INFINITY);
         bool ok = std::isfinite(pf);
         int lo[8] = {0}, hi[8] = {0};
-        for (size_t c = 0; ok && c < kids.size(); c++) {
-            lo[c] = (int)std::floor((kids[c].first - (double)pf) / s) - 1;
-            hi[c] = (int)std::ceil((kids[c].second - (double)pf) / s) + 1;
+        for (int c = 0; ok && c < n; c++) {
+            lo[c] = (int)std::floor(((double)kids[c].mn[axis] - (double)pf) / s) - 1;
+            hi[c] = (int)std::ceil(((double)kids[c].mx[axis] - (double)pf) / s) + 1;
             ok = lo[c] >= 0 && hi[c] <= 255;
         }
         if (!ok) continue;
         *p = pf;
         *e = (uint8_t)(k + 127);
-        for (size_t c = 0; c < 8; c++) {
-            qlo[c] = c < kids.size() ? (uint8_t)lo[c] : 255;    /* empty slots: lo > hi, never hit */
-            qhi[c] = c < kids.size() ? (uint8_t)hi[c] : 0;
+        for (int c = 0; c < 8; c++) {
+            qlo[c] = c < n ? (uint8_t)lo[c] : 255;    /* empty slots: lo > hi, never hit */
+            qhi[c] = c < n ? (uint8_t)hi[c] : 0;
         }
         return;
     }
@@ -235,53 +254,100 @@ static void quantise_axis(double mn, double mx, const std::vector<std::pair<doub
     for (int c = 0; c < 8; c++) { qlo[c] = 0; qhi[c] = 255; }
 }
 
+namespace {
+
+/* one wide node still to build: its binary node, its index among the nodes
+ * being built, and the stack entries that a traversal can hold above it */
+struct WideWork { int bnode, wnode, push; };
+
+/* Builds work.back()'s node into `nodes` and appends its interior children to
+ * both lists. */
+void wide_step(const Array<FlatNode>& fn, Array<WideNode>& nodes, std::vector<WideWork>& work, int* max_push) {
+    const WideWork w = work.back();
+    work.pop_back();
+    int kids[8] = {w.bnode + 1, fn[w.bnode].second}, n = 2;
+    float area[8];
+    for (int i = 0; i < 2; i++) area[i] = surface_area(fn[kids[i]].bounds);
+    while (n < 8) {
+        int best = -1;
+        float best_a = -1.0f;
+        for (int i = 0; i < n; i++)
+            if (fn[kids[i]].count == 0 && area[i] > best_a) { best_a = area[i]; best = i; }
+        if (best < 0) break;
+        for (int i = n; i > best + 1; i--) { kids[i] = kids[i - 1]; area[i] = area[i - 1]; }
+        const int b = kids[best];
+        kids[best] = b + 1;
+        kids[best + 1] = fn[b].second;
+        for (int i = best; i < best + 2; i++) area[i] = surface_area(fn[kids[i]].bounds);
+        n++;
+    }
+    Box kb[8];
+    for (int i = 0; i < n; i++) kb[i] = fn[kids[i]].bounds;
+    const Box& nb = fn[w.bnode].bounds;
+    WideNode d;
+    std::memset(&d, 0, sizeof(d));
+    d.nchild = (uint8_t)n;
+    for (int a = 0; a < 3; a++) quantise_axis((double)nb.mn[a], (double)nb.mx[a], kb, n, a, &d.p[a], &d.e[a], d.qlo[a], d.qhi[a]);
+    const int push = w.push + n - 1;
+    *max_push = std::max(*max_push, w.push);
+    for (int i = 0; i < 8; i++) { d.child[i] = i < n ? kids[i] : -1; d.wchild[i] = -1; }
+    for (int i = 0; i < n; i++) {
+        if (fn[kids[i]].count != 0) continue;
+        const int wi = (int)nodes.size();
+        d.wchild[i] = wi;
+        nodes.emplace_back();
+        work.push_back({kids[i], wi, push});
+    }
+    nodes[w.wnode] = d;
+}
+
+}  // namespace
+
 WideResult build_wide(const BuildResult& br) {
     WideResult r;
-    const std::vector<FlatNode>& fn = br.nodes;
+    const Array<FlatNode>& fn = br.nodes;
     if (fn.empty() || fn[0].count != 0) return r;
-    struct Work { int bnode, wnode, push; };
-    std::vector<Work> work{{0, 0, 0}};
+    /* the top of the tree here, breadth first, until it has enough subtrees for the host's cores */
+    std::vector<WideWork> work{{0, 0, 0}};
     r.nodes.emplace_back();
-    while (!work.empty()) {
-        const Work w = work.back();
-        work.pop_back();
-        std::vector<int> kids{w.bnode + 1, fn[w.bnode].second};
-        while (kids.size() < 8) {
-            int best = -1;
-            float best_a = -1.0f;
-            for (size_t i = 0; i < kids.size(); i++) {
-                if (fn[kids[i]].count != 0) continue;
-                const float a = surface_area(fn[kids[i]].bounds);
-                if (a > best_a) { best_a = a; best = (int)i; }
-            }
-            if (best < 0) break;
-            const int b = kids[best];
-            kids[best] = b + 1;
-            kids.insert(kids.begin() + best + 1, fn[b].second);
+    const size_t want = fn.size() > 8192 ? 128 : SIZE_MAX;
+    while (!work.empty() && work.size() < want) {
+        std::vector<WideWork> next;
+        while (!work.empty()) {
+            std::vector<WideWork> one{work.back()};
+            work.pop_back();
+            wide_step(fn, r.nodes, one, &r.max_push);
+            next.insert(next.end(), one.begin(), one.end());
         }
-        WideNode& n = r.nodes[w.wnode];
-        std::memset(&n, 0, sizeof(n));
-        n.nchild = (uint8_t)kids.size();
-        const Box& nb = fn[w.bnode].bounds;
-        for (int a = 0; a < 3; a++) {
-            std::vector<std::pair<double, double>> iv;
-            for (int k : kids) iv.emplace_back((double)fn[k].bounds.mn[a], (double)fn[k].bounds.mx[a]);
-            quantise_axis((double)nb.mn[a], (double)nb.mx[a], iv, &n.p[a], &n.e[a], n.qlo[a], n.qhi[a]);
-        }
-        const int push = w.push + (int)kids.size() - 1;
-        r.max_push = std::max(r.max_push, w.push);
-        for (size_t i = 0; i < 8; i++) {
-            n.child[i] = i < kids.size() ? kids[i] : -1;
-            n.wchild[i] = -1;
-        }
-        for (size_t i = 0; i < kids.size(); i++) {
-            if (fn[kids[i]].count != 0) continue;
-            const int wi = (int)r.nodes.size();
-            r.nodes[w.wnode].wchild[i] = wi;     /* r.nodes may reallocate below: index, not the reference */
-            r.nodes.emplace_back();
-            work.push_back({kids[i], wi, push});
-        }
+        work.swap(next);
     }
+    /* the subtrees, each into nodes of its own with its root first, then put after one another */
+    const size_t top = r.nodes.size(), subs = work.size();
+    std::vector<Array<WideNode>> sub(subs);
+    std::vector<int> push(subs, 0);
+    std::atomic<size_t> ticket{0};
+    parallel_for((int64_t)subs, 1, [&](int64_t, int64_t) {
+        for (size_t i = ticket++; i < subs; i = ticket++) {
+            std::vector<WideWork> todo{{work[i].bnode, 0, work[i].push}};
+            sub[i].emplace_back();
+            while (!todo.empty()) wide_step(fn, sub[i], todo, &push[i]);
+        }
+    });
+    std::vector<size_t> base(subs + 1, top);
+    for (size_t i = 0; i < subs; i++) {
+        base[i + 1] = base[i] + sub[i].size() - 1;               /* a subtree's root has its place already */
+        r.max_push = std::max(r.max_push, push[i]);
+    }
+    r.nodes.resize(base[subs]);
+    parallel_for((int64_t)subs, 1, [&](int64_t i0, int64_t i1) {
+        for (int64_t i = i0; i < i1; i++)
+            for (size_t k = 0; k < sub[i].size(); k++) {
+                WideNode& d = r.nodes[k == 0 ? (size_t)work[i].wnode : base[i] + k - 1];
+                d = sub[i][k];
+                for (int c = 0; c < 8; c++)
+                    if (d.wchild[c] >= 0) d.wchild[c] += (int)base[i] - 1;
+            }
+    });
     return r;
 }
 

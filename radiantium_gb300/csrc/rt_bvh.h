@@ -14,6 +14,7 @@
 
 #include <stdint.h>
 #include <vector>
+#include "rt_parallel.h"
 
 namespace rtb {
 
@@ -33,13 +34,13 @@ struct FlatNode {
 };
 
 struct BuildResult {
-    std::vector<FlatNode> nodes;
-    std::vector<int32_t> order;   /* slot -> primitive index */
+    Array<FlatNode> nodes;
+    Array<int32_t> order;         /* slot -> primitive index */
     int max_depth = 0;
 };
 
 /* prim_bounds: n boxes in primitive-list order */
-BuildResult build_sah(const std::vector<Box>& prim_bounds, int max_prims, int threads);
+BuildResult build_sah(const Array<Box>& prim_bounds, int max_prims, int threads);
 
 /* An 8-wide node of the wide tree that the opt-in fast traversal reads: up to
  * eight children of the binary tree collapsed into one node (the interior
@@ -58,7 +59,7 @@ struct WideNode {
 };
 
 struct WideResult {
-    std::vector<WideNode> nodes;     /* nodes[0] is the root when the binary root is interior */
+    Array<WideNode> nodes;           /* nodes[0] is the root when the binary root is interior */
     int max_push = 0;                /* most stack entries a traversal can hold below any node */
 };
 

@@ -25,6 +25,7 @@
 
 #include "rt_bvh.h"
 #include "rt_bvh_gpu.h"
+#include <memory>
 
 namespace {
 
@@ -430,7 +431,7 @@ void scan(int* a, int n, int* bsum, cudaStream_t s) {
 
 #define GK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { err = e_; goto done; } } while (0)
 
-cudaError_t rt_gpu_build_sah(const std::vector<rtb::Box>& bounds, int max_prims, rtb::BuildResult* out,
+cudaError_t rt_gpu_build_sah(const rtb::Array<rtb::Box>& bounds, int max_prims, rtb::BuildResult* out,
                              cudaStream_t s) {
     cudaError_t err = cudaSuccess;
     const int n = (int)bounds.size();
@@ -440,30 +441,32 @@ cudaError_t rt_gpu_build_sah(const std::vector<rtb::Box>& bounds, int max_prims,
     Dev D;
     D.n = n;
     float* d_box = nullptr;
-    std::vector<GNode> hn;
-    std::vector<int> perm;
+    char* arena = nullptr;
+    std::unique_ptr<GNode[]> hn;
     std::vector<int> level_start;       /* first BFS node id of every level */
     int nodes_used = 1, nseg = 1;
     const int max_nodes = 2 * n;
     const int nbs = (n + 1023) / 1024 + 2;
-    GK(rt_dev_malloc((void**)&d_box, (size_t)n * 6 * sizeof(float)));
+    /* every array in one allocation */
+    {
+        struct Part { void** p; size_t bytes; };
+        const Part parts[] = {
+            {(void**)&d_box, (size_t)n * 6 * sizeof(float)}, {(void**)&D.cent, (size_t)n * 3 * sizeof(float)},
+            {(void**)&D.perm, (size_t)n * sizeof(int)}, {(void**)&D.perm2, (size_t)n * sizeof(int)},
+            {(void**)&D.item_seg, (size_t)n * sizeof(int)}, {(void**)&D.fflag, (size_t)(n + 1) * sizeof(int)},
+            {(void**)&D.tflag, (size_t)(n + 1) * sizeof(int)}, {(void**)&D.fpos, (size_t)n * sizeof(int)},
+            {(void**)&D.tpos, (size_t)n * sizeof(int)}, {(void**)&D.bsum, (size_t)nbs * sizeof(int)},
+            {(void**)&D.seg, (size_t)n * sizeof(Seg)}, {(void**)&D.seg2, (size_t)n * sizeof(Seg)},
+            {(void**)&D.acc, (size_t)n * sizeof(SegAcc)}, {(void**)&D.plan, (size_t)n * sizeof(SegPlan)},
+            {(void**)&D.split, (size_t)(n + 1) * sizeof(int)}, {(void**)&D.nodes, (size_t)max_nodes * sizeof(GNode)}};
+        size_t total = 0;
+        for (const Part& q : parts) total += (q.bytes + 255) & ~(size_t)255;
+        GK(rt_dev_malloc((void**)&arena, total));
+        char* at = arena;
+        for (const Part& q : parts) { *q.p = at; at += (q.bytes + 255) & ~(size_t)255; }
+    }
     GK(cudaMemcpyAsync(d_box, bounds.data(), (size_t)n * 6 * sizeof(float), cudaMemcpyHostToDevice, s));
     D.box = d_box;
-    GK(rt_dev_malloc((void**)&D.cent, (size_t)n * 3 * sizeof(float)));
-    GK(rt_dev_malloc((void**)&D.perm, (size_t)n * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.perm2, (size_t)n * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.item_seg, (size_t)n * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.fflag, (size_t)(n + 1) * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.tflag, (size_t)(n + 1) * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.fpos, (size_t)n * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.tpos, (size_t)n * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.bsum, (size_t)nbs * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.seg, (size_t)n * sizeof(Seg)));
-    GK(rt_dev_malloc((void**)&D.seg2, (size_t)n * sizeof(Seg)));
-    GK(rt_dev_malloc((void**)&D.acc, (size_t)n * sizeof(SegAcc)));
-    GK(rt_dev_malloc((void**)&D.plan, (size_t)n * sizeof(SegPlan)));
-    GK(rt_dev_malloc((void**)&D.split, (size_t)(n + 1) * sizeof(int)));
-    GK(rt_dev_malloc((void**)&D.nodes, (size_t)max_nodes * sizeof(GNode)));
     k_init<<<gridn(n, 256), 256, 0, s>>>(D);
     {
         const Seg root{0, n, 0, 0};
@@ -499,10 +502,10 @@ cudaError_t rt_gpu_build_sah(const std::vector<rtb::Box>& bounds, int max_prims,
         nseg = next;
     }
     /* depth-first flattening on the host from the BFS records */
-    hn.resize(nodes_used);
-    perm.resize(n);
-    GK(cudaMemcpyAsync(hn.data(), D.nodes, (size_t)nodes_used * sizeof(GNode), cudaMemcpyDeviceToHost, s));
-    GK(cudaMemcpyAsync(perm.data(), D.perm, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, s));
+    hn.reset(new GNode[nodes_used]);
+    out->order.resize(n);
+    GK(cudaMemcpyAsync(hn.get(), D.nodes, (size_t)nodes_used * sizeof(GNode), cudaMemcpyDeviceToHost, s));
+    GK(cudaMemcpyAsync(out->order.data(), D.perm, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, s));
     GK(cudaStreamSynchronize(s));
     GK(cudaGetLastError());
     {
@@ -515,18 +518,17 @@ cudaError_t rt_gpu_build_sah(const std::vector<rtb::Box>& bounds, int max_prims,
                 dfs[hn[v].right] = dfs[v] + 1 + size[hn[v].left];
             }
         out->nodes.resize(nodes_used);
-        for (int v = 0; v < nodes_used; v++) {
-            rtb::FlatNode& f = out->nodes[dfs[v]];
-            for (int k = 0; k < 3; k++) { f.bounds.mn[k] = hn[v].mn[k]; f.bounds.mx[k] = hn[v].mx[k]; }
-            if (hn[v].left >= 0) { f.second = dfs[hn[v].right]; f.count = 0; f.axis = hn[v].axis; }
-            else { f.second = hn[v].lo; f.count = hn[v].count; f.axis = 0; }
-        }
-        out->order.assign(perm.begin(), perm.end());
+        rtb::parallel_for(nodes_used, 16384, [&](int64_t v0, int64_t v1) {
+            for (int64_t v = v0; v < v1; v++) {
+                rtb::FlatNode& f = out->nodes[dfs[v]];
+                for (int k = 0; k < 3; k++) { f.bounds.mn[k] = hn[v].mn[k]; f.bounds.mx[k] = hn[v].mx[k]; }
+                if (hn[v].left >= 0) { f.second = dfs[hn[v].right]; f.count = 0; f.axis = hn[v].axis; }
+                else { f.second = hn[v].lo; f.count = hn[v].count; f.axis = 0; }
+            }
+        });
         out->max_depth = (int)level_start.size() - 1;
     }
 done:
-    cudaFree(d_box); cudaFree(D.cent); cudaFree(D.perm); cudaFree(D.perm2); cudaFree(D.item_seg);
-    cudaFree(D.fflag); cudaFree(D.tflag); cudaFree(D.fpos); cudaFree(D.tpos); cudaFree(D.bsum);
-    cudaFree(D.seg); cudaFree(D.seg2); cudaFree(D.acc); cudaFree(D.plan); cudaFree(D.split); cudaFree(D.nodes);
+    cudaFree(arena);
     return err;
 }

@@ -12,6 +12,6 @@
  * so tests can show which entry points allocate device memory */
 cudaError_t rt_dev_malloc(void** p, size_t bytes);
 
-cudaError_t rt_gpu_build_sah(const std::vector<rtb::Box>& bounds, int max_prims, rtb::BuildResult* out, cudaStream_t s);
+cudaError_t rt_gpu_build_sah(const rtb::Array<rtb::Box>& bounds, int max_prims, rtb::BuildResult* out, cudaStream_t s);
 
 #endif

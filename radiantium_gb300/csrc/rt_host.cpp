@@ -146,8 +146,8 @@ void ensure_events(Ctx* c, size_t n) {
     }
 }
 
-template <class T>
-T* upload(Ctx* c, const std::vector<T>& v) {
+template <class T, class A>
+T* upload(Ctx* c, const std::vector<T, A>& v) {
     DevBuf b;
     b.bytes = std::max<size_t>(sizeof(T), v.size() * sizeof(T));
     CK(rt_dev_malloc(&b.p, b.bytes));
@@ -356,7 +356,7 @@ void check_index(int i, int n, const char* what) {
 /* builds one BVH; appends nodes and slots; fills the header */
 /* The reference's SAH tree: on the GPU for large primitive counts (the same
  * tree, rt_bvh_gpu.cu), on the host threads otherwise. */
-rtb::BuildResult build_tree(Ctx* c, const std::vector<rtb::Box>& boxes, int maxp, int threads) {
+rtb::BuildResult build_tree(Ctx* c, const rtb::Array<rtb::Box>& boxes, int maxp, int threads) {
     if ((int64_t)boxes.size() >= c->gpu_build_min) {
         rtb::BuildResult r;
         CK(rt_gpu_build_sah(boxes, maxp, &r, c->stream));
@@ -368,32 +368,35 @@ rtb::BuildResult build_tree(Ctx* c, const std::vector<rtb::Box>& boxes, int maxp
 /* the wide form of a tree (rtb::build_wide) for the fast traversal; leaf refs
  * are the binary tree's (first slot, count in that slot).  Returns the most
  * stack entries a wide traversal of the tree can hold below a node. */
-int emit_wide(const rtb::BuildResult& br, int slot_base, std::vector<float4>& wnodes, RtBvh* hdr) {
-    const std::vector<rtb::FlatNode>& fn = br.nodes;
+int emit_wide(const rtb::BuildResult& br, int slot_base, rtb::Array<float4>& wnodes, RtBvh* hdr) {
+    const rtb::Array<rtb::FlatNode>& fn = br.nodes;
     if (fn.empty()) { hdr->wide_root = INT_MIN; return 0; }
     if (fn[0].count != 0) { hdr->wide_root = hdr->root_ref; return 0; }
     const rtb::WideResult w = rtb::build_wide(br);
     const int base = (int)(wnodes.size() / RT_WIDE_F4);
     hdr->wide_root = base;
-    for (const rtb::WideNode& n : w.nodes) {
-        uint32_t meta = (uint32_t)n.e[0] | ((uint32_t)n.e[1] << 8) | ((uint32_t)n.e[2] << 16) | ((uint32_t)n.nchild << 24);
-        float4 f[RT_WIDE_F4];
-        f[0] = make_float4(n.p[0], n.p[1], n.p[2], 0.0f);
-        std::memcpy(&f[0].w, &meta, 4);
-        for (int a = 0; a < 3; a++) {
-            std::memcpy(&f[1 + a].x, n.qlo[a], 8);
-            std::memcpy(&f[1 + a].z, n.qhi[a], 8);
+    wnodes.resize((size_t)(base + (int64_t)w.nodes.size()) * RT_WIDE_F4);
+    rtb::parallel_for((int64_t)w.nodes.size(), 4096, [&](int64_t i0, int64_t i1) {
+        for (int64_t i = i0; i < i1; i++) {
+            const rtb::WideNode& n = w.nodes[i];
+            uint32_t meta = (uint32_t)n.e[0] | ((uint32_t)n.e[1] << 8) | ((uint32_t)n.e[2] << 16) | ((uint32_t)n.nchild << 24);
+            float4* f = &wnodes[(size_t)(base + i) * RT_WIDE_F4];
+            f[0] = make_float4(n.p[0], n.p[1], n.p[2], 0.0f);
+            std::memcpy(&f[0].w, &meta, 4);
+            for (int a = 0; a < 3; a++) {
+                std::memcpy(&f[1 + a].x, n.qlo[a], 8);
+                std::memcpy(&f[1 + a].z, n.qhi[a], 8);
+            }
+            int32_t ref[8];
+            for (int k = 0; k < 8; k++) {
+                if (k >= n.nchild) ref[k] = INT_MIN;
+                else if (n.wchild[k] >= 0) ref[k] = base + n.wchild[k];
+                else ref[k] = ~(slot_base + fn[n.child[k]].second);
+            }
+            std::memcpy(&f[4], ref, 16);
+            std::memcpy(&f[5], ref + 4, 16);
         }
-        int32_t ref[8];
-        for (int k = 0; k < 8; k++) {
-            if (k >= n.nchild) ref[k] = INT_MIN;
-            else if (n.wchild[k] >= 0) ref[k] = base + n.wchild[k];
-            else ref[k] = ~(slot_base + fn[n.child[k]].second);
-        }
-        std::memcpy(&f[4], ref, 16);
-        std::memcpy(&f[5], ref + 4, 16);
-        for (int q = 0; q < RT_WIDE_F4; q++) wnodes.push_back(f[q]);
-    }
+    });
     return w.max_push;
 }
 
@@ -404,49 +407,54 @@ bool inverted(const rtb::Box& b) {
 }
 
 /* returns whether a box is inverted */
-bool emit_bvh(const rtb::BuildResult& br, const std::vector<std::array<float4, 3>>& recs, std::vector<float4>& nodes,
-              std::vector<float4>& slots, RtBvh* hdr) {
+bool emit_bvh(const rtb::BuildResult& br, const rtb::Array<std::array<float4, 3>>& recs, rtb::Array<float4>& nodes,
+              rtb::Array<float4>& slots, RtBvh* hdr) {
     const int slot_base = (int)(slots.size() / 3);
-    for (size_t i = 0; i < br.order.size(); i++) {
-        const std::array<float4, 3>& r = recs[br.order[i]];
-        slots.push_back(r[0]); slots.push_back(r[1]); slots.push_back(r[2]);
-    }
-    const std::vector<rtb::FlatNode>& fn = br.nodes;
+    slots.resize(slots.size() + 3 * br.order.size());
+    rtb::parallel_for((int64_t)br.order.size(), 16384, [&](int64_t i0, int64_t i1) {
+        for (int64_t i = i0; i < i1; i++) {
+            const std::array<float4, 3>& r = recs[br.order[i]];
+            for (int k = 0; k < 3; k++) slots[3 * (slot_base + (size_t)i) + k] = r[k];
+        }
+    });
+    const rtb::Array<rtb::FlatNode>& fn = br.nodes;
     if (fn.empty()) {
         for (int k = 0; k < 3; k++) { hdr->root_min[k] = 0; hdr->root_max[k] = 0; }
         hdr->root_ref = INT_MIN;
         return false;
     }
-    bool odd = inverted(fn[0].bounds);
     /* interior nodes get consecutive device indices in depth-first order */
     std::vector<int> dev(fn.size(), -1);
-    int node_base = (int)(nodes.size() / 4), nint = 0;
-    for (size_t i = 0; i < fn.size(); i++) if (fn[i].count == 0) dev[i] = node_base + nint++;
-    auto ref_of = [&](int i) -> int {
-        if (fn[i].count == 0) return dev[i];
-        int first = slot_base + fn[i].second;
-        if (fn[i].count > 65535) throw RtFail(RT_ERR_UNSUPPORTED, "BVH leaf with more than 65535 primitives");
-        float4& s2 = slots[3 * (size_t)first + 2];
-        int c = fn[i].count;
-        std::memcpy(&s2.w, &c, 4);
-        return ~first;
-    };
+    const int node_base = (int)(nodes.size() / 4);
+    int nint = 0;
+    for (size_t i = 0; i < fn.size(); i++) {
+        if (fn[i].count == 0) dev[i] = node_base + nint++;
+        else if (fn[i].count > 65535) throw RtFail(RT_ERR_UNSUPPORTED, "BVH leaf with more than 65535 primitives");
+    }
+    auto ref_of = [&](int i) -> int { return fn[i].count == 0 ? dev[i] : ~(slot_base + fn[i].second); };
     for (int k = 0; k < 3; k++) { hdr->root_min[k] = fn[0].bounds.mn[k]; hdr->root_max[k] = fn[0].bounds.mx[k]; }
     hdr->root_ref = ref_of(0);
-    for (size_t i = 0; i < fn.size(); i++) {
-        if (fn[i].count != 0) { ref_of((int)i); continue; }
-        const rtb::Box& L = fn[i + 1].bounds;
-        const rtb::Box& R = fn[fn[i].second].bounds;
-        odd = odd || inverted(L) || inverted(R);
-        int lref = ref_of((int)i + 1), rref = ref_of(fn[i].second), axis = fn[i].axis;
-        float4 n0 = make_float4(L.mn[0], R.mn[0], L.mx[0], R.mx[0]);
-        float4 n1 = make_float4(L.mn[1], R.mn[1], L.mx[1], R.mx[1]);
-        float4 n2 = make_float4(L.mn[2], R.mn[2], L.mx[2], R.mx[2]);
-        float4 n3;
-        std::memcpy(&n3.x, &lref, 4); std::memcpy(&n3.y, &rref, 4); std::memcpy(&n3.z, &axis, 4); n3.w = 0;
-        nodes.push_back(n0); nodes.push_back(n1); nodes.push_back(n2); nodes.push_back(n3);
-    }
-    return odd;
+    std::atomic<bool> odd{inverted(fn[0].bounds)};
+    nodes.resize((size_t)(node_base + (int64_t)nint) * 4);
+    rtb::parallel_for((int64_t)fn.size(), 16384, [&](int64_t i0, int64_t i1) {
+        bool o = false;
+        for (int64_t i = i0; i < i1; i++) {
+            if (fn[i].count != 0) {              /* a leaf: its count goes to its first slot */
+                const int c = fn[i].count;
+                std::memcpy(&slots[3 * (size_t)(slot_base + fn[i].second) + 2].w, &c, 4);
+                continue;
+            }
+            const rtb::Box& L = fn[i + 1].bounds;
+            const rtb::Box& R = fn[fn[i].second].bounds;
+            o = o || inverted(L) || inverted(R);
+            const int lref = ref_of((int)i + 1), rref = ref_of(fn[i].second), axis = fn[i].axis;
+            float4* n = &nodes[4 * (size_t)dev[i]];
+            for (int a = 0; a < 3; a++) n[a] = make_float4(L.mn[a], R.mn[a], L.mx[a], R.mx[a]);
+            std::memcpy(&n[3].x, &lref, 4); std::memcpy(&n[3].y, &rref, 4); std::memcpy(&n[3].z, &axis, 4); n[3].w = 0;
+        }
+        if (o) odd.store(true);
+    });
+    return odd.load();
 }
 
 inline float4 f4bits(float x, float y, float z, int w) { float4 r = make_float4(x, y, z, 0); std::memcpy(&r.w, &w, 4); return r; }
@@ -471,6 +479,19 @@ rtb::Box tri_box(const rt_mesh_desc& m, int t) {
     float q[3] = {pb.x, pb.y, pb.z}; rtb::box_expand(b, q);
     float r[3] = {pc.x, pc.y, pc.z}; rtb::box_expand(b, r);
     return b;
+}
+/* the mesh's triangles, as primitives first_id and on and global triangles first_tri and on */
+void append_mesh(const rt_mesh_desc& m, int first_tri, int first_id, rtb::Array<rtb::Box>& boxes,
+                 rtb::Array<std::array<float4, 3>>& recs) {
+    const size_t b0 = boxes.size(), r0 = recs.size();
+    boxes.resize(b0 + m.triangle_count);
+    recs.resize(r0 + m.triangle_count);
+    rtb::parallel_for(m.triangle_count, 16384, [&](int64_t i0, int64_t i1) {
+        for (int64_t t = i0; t < i1; t++) {
+            boxes[b0 + t] = tri_box(m, (int)t);
+            recs[r0 + t] = tri_rec(m, (int)t, first_id + (int)t, first_tri + (int)t);
+        }
+    });
 }
 rtb::Box sphere_box(const rt_sphere_desc& s) {
     rtb::Box b;
@@ -498,9 +519,9 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
     int tallest = 0;                           /* levels of the tallest tree */
 
     /* global vertex / triangle tables: every mesh, in mesh order */
-    std::vector<float4> pos, nrm;
-    std::vector<float2> uvs;
-    std::vector<RtTri> tris;
+    rtb::Array<float4> pos, nrm;
+    rtb::Array<float2> uvs;
+    rtb::Array<RtTri> tris;
     std::vector<int> mesh_tri_base(d->mesh_count), mesh_vtx_base(d->mesh_count);
     for (int m = 0; m < d->mesh_count; m++) {
         const rt_mesh_desc& md = d->meshes[m];
@@ -508,23 +529,29 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
             throw RtFail(RT_ERR_INVALID_ARG, "scene: mesh " + std::to_string(m) + " has no positions / indices");
         mesh_vtx_base[m] = (int)pos.size();
         mesh_tri_base[m] = (int)tris.size();
-        for (int i = 0; i < md.vertex_count; i++) {
-            pos.push_back(make_float4(md.positions[3 * i], md.positions[3 * i + 1], md.positions[3 * i + 2], 0));
-            nrm.push_back(md.normals ? make_float4(md.normals[3 * i], md.normals[3 * i + 1], md.normals[3 * i + 2], 0) : make_float4(0, 0, 0, 0));
-            uvs.push_back(md.uvs ? make_float2(md.uvs[2 * i], md.uvs[2 * i + 1]) : make_float2(0, 0));
-        }
-        for (int t = 0; t < md.triangle_count; t++) {
-            RtTri tr;
-            for (int k = 0; k < 3; k++) {
-                int vi = md.indices[3 * t + k];
-                if (vi < 0 || vi >= md.vertex_count) throw RtFail(RT_ERR_INVALID_ARG, "scene: mesh " + std::to_string(m) + " index out of range");
+        const size_t v0 = pos.size(), t0 = tris.size();
+        pos.resize(v0 + md.vertex_count);
+        nrm.resize(v0 + md.vertex_count);
+        uvs.resize(v0 + md.vertex_count);
+        rtb::parallel_for(md.vertex_count, 16384, [&](int64_t i0, int64_t i1) {
+            for (int64_t i = i0; i < i1; i++) {
+                pos[v0 + i] = make_float4(md.positions[3 * i], md.positions[3 * i + 1], md.positions[3 * i + 2], 0);
+                nrm[v0 + i] = md.normals ? make_float4(md.normals[3 * i], md.normals[3 * i + 1], md.normals[3 * i + 2], 0) : make_float4(0, 0, 0, 0);
+                uvs[v0 + i] = md.uvs ? make_float2(md.uvs[2 * i], md.uvs[2 * i + 1]) : make_float2(0, 0);
             }
-            tr.v0 = mesh_vtx_base[m] + md.indices[3 * t];
-            tr.v1 = mesh_vtx_base[m] + md.indices[3 * t + 1];
-            tr.v2 = mesh_vtx_base[m] + md.indices[3 * t + 2];
-            tr.flags = (md.normals ? 1 : 0) | (md.uvs ? 2 : 0);
-            tris.push_back(tr);
-        }
+        });
+        tris.resize(t0 + md.triangle_count);
+        std::atomic<bool> bad{false};
+        rtb::parallel_for(md.triangle_count, 16384, [&](int64_t i0, int64_t i1) {
+            const int flags = (md.normals ? 1 : 0) | (md.uvs ? 2 : 0), base = (int)v0;
+            for (int64_t t = i0; t < i1; t++) {
+                const int* ix = md.indices + 3 * t;
+                for (int k = 0; k < 3; k++)
+                    if (ix[k] < 0 || ix[k] >= md.vertex_count) { bad.store(true); return; }
+                tris[t0 + t] = RtTri{base + ix[0], base + ix[1], base + ix[2], flags};
+            }
+        });
+        if (bad.load()) throw RtFail(RT_ERR_INVALID_ARG, "scene: mesh " + std::to_string(m) + " index out of range");
     }
     std::vector<RtSphere> spheres(d->sphere_count);
     for (int i = 0; i < d->sphere_count; i++) {
@@ -543,17 +570,17 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
             throw RtFail(RT_ERR_INVALID_ARG, "scene: material " + std::to_string(i) + " is missing a texture or has an unknown type");
     }
 
-    std::vector<float4> nodes, slots, wnodes;
+    rtb::Array<float4> nodes, slots, wnodes;
     int wide_push = 0;
     bool odd_boxes = false;                    /* a box with min > max */
     std::vector<RtBvh> bvhs(1 + d->blas_count);
     /* instanced prototypes: ShapeWrapperPrimitive per shape (RendererBuilder.cs:895-921) */
-    std::vector<rtb::Box> blas_root(d->blas_count);
+    rtb::Array<rtb::Box> blas_root(d->blas_count);
     for (int b = 0; b < d->blas_count; b++) {
         int first = d->blas_ranges[2 * b], count = d->blas_ranges[2 * b + 1];
         if (first < 0 || count < 0 || first + count > d->blas_group_count) throw RtFail(RT_ERR_INVALID_ARG, "scene: bad prototype range");
-        std::vector<rtb::Box> boxes;
-        std::vector<std::array<float4, 3>> recs;
+        rtb::Array<rtb::Box> boxes;
+        rtb::Array<std::array<float4, 3>> recs;
         for (int g = first; g < first + count; g++) {
             const rt_group_desc& gd = d->blas_groups[g];
             if (gd.kind == RT_GROUP_SPHERE) {
@@ -563,10 +590,7 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
             } else if (gd.kind == RT_GROUP_MESH) {
                 check_index(gd.ref, d->mesh_count, "mesh");
                 const rt_mesh_desc& md = d->meshes[gd.ref];
-                for (int t = 0; t < md.triangle_count; t++) {
-                    boxes.push_back(tri_box(md, t));
-                    recs.push_back(tri_rec(md, t, (int)recs.size(), mesh_tri_base[gd.ref] + t));
-                }
+                append_mesh(md, mesh_tri_base[gd.ref], (int)recs.size(), boxes, recs);
             } else {
                 throw RtFail(RT_ERR_INVALID_ARG, "scene: instanced prototype groups must be meshes or spheres");
             }
@@ -581,9 +605,9 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
     }
 
     /* top level, lights, infinite lights */
-    std::vector<rtb::Box> boxes;
-    std::vector<std::array<float4, 3>> recs;
-    std::vector<RtPrim> prims;
+    rtb::Array<rtb::Box> boxes;
+    rtb::Array<std::array<float4, 3>> recs;
+    rtb::Array<RtPrim> prims;
     std::vector<RtLight> lights;
     std::vector<int32_t> infinite;
     std::vector<RtInstance> insts;
@@ -625,20 +649,21 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
         case RT_GROUP_MESH: {
             check_index(gd.ref, d->mesh_count, "mesh");
             const rt_mesh_desc& md = d->meshes[gd.ref];
-            for (int t = 0; t < md.triangle_count; t++) {
-                int id = (int)prims.size();
-                int gt = mesh_tri_base[gd.ref] + t;
-                int li = -1;
-                if (gd.emissive) {
+            const size_t id = prims.size();
+            const int gt = mesh_tri_base[gd.ref];
+            append_mesh(md, gt, (int)id, boxes, recs);
+            prims.resize(id + md.triangle_count);
+            rtb::parallel_for(md.triangle_count, 16384, [&](int64_t i0, int64_t i1) {
+                for (int64_t t = i0; t < i1; t++)
+                    prims[id + t] = RtPrim{RT_KIND_TRI, gt + (int)t, tp.material, -1, tp.med_in, tp.med_out, 0, 0};
+            });
+            if (gd.emissive)                     /* one light per triangle, in order */
+                for (int t = 0; t < md.triangle_count; t++) {
                     const int* ix = md.indices + 3 * (size_t)t;
                     F3 pa = vertex(md, ix[0]), pb = vertex(md, ix[1]), pc = vertex(md, ix[2]);
                     float area = 0.5f * length(cross(sub(pb, pa), sub(pc, pa)));
-                    li = area_light(RT_LIGHT_AREA_TRI, gt, gd, area);
+                    prims[id + t].light = area_light(RT_LIGHT_AREA_TRI, gt + t, gd, area);
                 }
-                prims.push_back(RtPrim{RT_KIND_TRI, gt, tp.material, li, tp.med_in, tp.med_out, 0, 0});
-                boxes.push_back(tri_box(md, t));
-                recs.push_back(tri_rec(md, t, id, gt));
-            }
             break;
         }
         case RT_GROUP_INSTANCE: {
@@ -1925,7 +1950,7 @@ int rt_debug_bvh(const float* boxes, int n, int max_prims, int64_t* node_count, 
                  int32_t* count, int32_t* axis, int32_t* order) {
     if (!boxes || n <= 0 || !node_count) return RT_ERR_INVALID_ARG;
     try {
-        std::vector<rtb::Box> b(n);
+        rtb::Array<rtb::Box> b(n);
         for (int i = 0; i < n; i++)
             for (int k = 0; k < 3; k++) { b[i].mn[k] = boxes[6 * i + k]; b[i].mx[k] = boxes[6 * i + 3 + k]; }
         rtb::BuildResult r = rtb::build_sah(b, max_prims, std::max(1u, std::thread::hardware_concurrency()));
@@ -1952,7 +1977,7 @@ int rt_debug_wide(const float* boxes, int n, int max_prims, int64_t* node_count,
                   uint8_t* qlo, uint8_t* qhi, int32_t* child, int32_t* wchild, int32_t* max_push) {
     if (!boxes || n <= 0 || !node_count) return RT_ERR_INVALID_ARG;
     try {
-        std::vector<rtb::Box> b(n);
+        rtb::Array<rtb::Box> b(n);
         for (int i = 0; i < n; i++)
             for (int k = 0; k < 3; k++) { b[i].mn[k] = boxes[6 * i + k]; b[i].mx[k] = boxes[6 * i + 3 + k]; }
         rtb::BuildResult r = rtb::build_sah(b, max_prims, std::max(1u, std::thread::hardware_concurrency()));
@@ -1984,7 +2009,7 @@ int rt_debug_bvh_gpu(void* ctx, const float* boxes, int n, int max_prims, int64_
     Ctx* c = (Ctx*)ctx;
     if (!boxes || n <= 0 || !node_count) return RT_ERR_INVALID_ARG;
     return run(c, [&]() {
-        std::vector<rtb::Box> b(n);
+        rtb::Array<rtb::Box> b(n);
         for (int i = 0; i < n; i++)
             for (int k = 0; k < 3; k++) { b[i].mn[k] = boxes[6 * i + k]; b[i].mx[k] = boxes[6 * i + 3 + k]; }
         rtb::BuildResult r;
