@@ -25,7 +25,6 @@
 
 #include "rt_bvh.h"
 #include "rt_bvh_gpu.h"
-#include <memory>
 
 namespace {
 
@@ -78,6 +77,8 @@ struct Dev {
     SegPlan* plan = nullptr;
     int* split = nullptr;        /* per segment: 2 if split, 0 leaf; scanned */
     GNode* nodes = nullptr;
+    int* size = nullptr; int* dfs = nullptr;      /* per node: nodes of its subtree, depth-first index */
+    rtb::FlatNode* flat = nullptr;               /* the nodes in depth-first order */
     int* meta = nullptr;         /* [0] nodes used */
 };
 
@@ -427,6 +428,36 @@ void scan(int* a, int n, int* bsum, cudaStream_t s) {
     k_scan_add<<<nb, 1024, 0, s>>>(a, n, bsum, nb);
 }
 
+/* flattening (the levels' nodes are consecutive): a level's subtree sizes, its
+ * children's depth-first indices, and every node's record */
+__global__ void k_sizes(Dev D, int v0, int v1) {
+    const int v = v0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= v1) return;
+    const GNode& nd = D.nodes[v];
+    D.size[v] = nd.left >= 0 ? 1 + D.size[nd.left] + D.size[nd.right] : 1;
+}
+__global__ void k_dfs(Dev D, int v0, int v1) {
+    const int v = v0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= v1) return;
+    if (v == 0) D.dfs[0] = 0;
+    const GNode& nd = D.nodes[v];
+    if (nd.left < 0) return;
+    const int at = v == 0 ? 0 : D.dfs[v];
+    D.dfs[nd.left] = at + 1;
+    D.dfs[nd.right] = at + 1 + D.size[nd.left];
+}
+__global__ void k_flatten(Dev D, int n) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    const GNode& nd = D.nodes[v];
+    rtb::FlatNode& f = D.flat[D.dfs[v]];
+    for (int k = 0; k < 3; k++) { f.bounds.mn[k] = nd.mn[k]; f.bounds.mx[k] = nd.mx[k]; }
+    const bool inner = nd.left >= 0;
+    f.second = inner ? D.dfs[nd.right] : nd.lo;
+    f.count = inner ? 0 : nd.count;
+    f.axis = inner ? nd.axis : 0;
+}
+
 }  // namespace
 
 #define GK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { err = e_; goto done; } } while (0)
@@ -442,7 +473,6 @@ cudaError_t rt_gpu_build_sah(const rtb::Array<rtb::Box>& bounds, int max_prims, 
     D.n = n;
     float* d_box = nullptr;
     char* arena = nullptr;
-    std::unique_ptr<GNode[]> hn;
     std::vector<int> level_start;       /* first BFS node id of every level */
     int nodes_used = 1, nseg = 1;
     const int max_nodes = 2 * n;
@@ -458,7 +488,9 @@ cudaError_t rt_gpu_build_sah(const rtb::Array<rtb::Box>& bounds, int max_prims, 
             {(void**)&D.tpos, (size_t)n * sizeof(int)}, {(void**)&D.bsum, (size_t)nbs * sizeof(int)},
             {(void**)&D.seg, (size_t)n * sizeof(Seg)}, {(void**)&D.seg2, (size_t)n * sizeof(Seg)},
             {(void**)&D.acc, (size_t)n * sizeof(SegAcc)}, {(void**)&D.plan, (size_t)n * sizeof(SegPlan)},
-            {(void**)&D.split, (size_t)(n + 1) * sizeof(int)}, {(void**)&D.nodes, (size_t)max_nodes * sizeof(GNode)}};
+            {(void**)&D.split, (size_t)(n + 1) * sizeof(int)}, {(void**)&D.nodes, (size_t)max_nodes * sizeof(GNode)},
+            {(void**)&D.size, (size_t)max_nodes * sizeof(int)}, {(void**)&D.dfs, (size_t)max_nodes * sizeof(int)},
+            {(void**)&D.flat, (size_t)max_nodes * sizeof(rtb::FlatNode)}};
         size_t total = 0;
         for (const Part& q : parts) total += (q.bytes + 255) & ~(size_t)255;
         GK(rt_dev_malloc((void**)&arena, total));
@@ -501,32 +533,23 @@ cudaError_t rt_gpu_build_sah(const rtb::Array<rtb::Box>& bounds, int max_prims, 
         nodes_used += next;
         nseg = next;
     }
-    /* depth-first flattening on the host from the BFS records */
-    hn.reset(new GNode[nodes_used]);
-    out->order.resize(n);
-    GK(cudaMemcpyAsync(hn.get(), D.nodes, (size_t)nodes_used * sizeof(GNode), cudaMemcpyDeviceToHost, s));
-    GK(cudaMemcpyAsync(out->order.data(), D.perm, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, s));
-    GK(cudaStreamSynchronize(s));
-    GK(cudaGetLastError());
+    /* depth-first flattening: subtree sizes from the last level up, depth-first
+     * indices from the first level down, then every node to its place */
     {
-        std::vector<int> size(nodes_used, 1), dfs(nodes_used, 0);
-        for (int v = nodes_used - 1; v >= 0; v--)
-            if (hn[v].left >= 0) size[v] = 1 + size[hn[v].left] + size[hn[v].right];
-        for (int v = 0; v < nodes_used; v++)         /* BFS order: parents before children */
-            if (hn[v].left >= 0) {
-                dfs[hn[v].left] = dfs[v] + 1;
-                dfs[hn[v].right] = dfs[v] + 1 + size[hn[v].left];
-            }
+        const int levels = (int)level_start.size() - 1;
+        auto span = [&](int l) { return level_start[l + 1] - level_start[l]; };
+        for (int l = levels - 1; l >= 0; l--)
+            k_sizes<<<gridn(span(l), 256), 256, 0, s>>>(D, level_start[l], level_start[l + 1]);
+        for (int l = 0; l < levels; l++)
+            k_dfs<<<gridn(span(l), 256), 256, 0, s>>>(D, level_start[l], level_start[l + 1]);
+        k_flatten<<<gridn(nodes_used, 256), 256, 0, s>>>(D, nodes_used);
         out->nodes.resize(nodes_used);
-        rtb::parallel_for(nodes_used, 16384, [&](int64_t v0, int64_t v1) {
-            for (int64_t v = v0; v < v1; v++) {
-                rtb::FlatNode& f = out->nodes[dfs[v]];
-                for (int k = 0; k < 3; k++) { f.bounds.mn[k] = hn[v].mn[k]; f.bounds.mx[k] = hn[v].mx[k]; }
-                if (hn[v].left >= 0) { f.second = dfs[hn[v].right]; f.count = 0; f.axis = hn[v].axis; }
-                else { f.second = hn[v].lo; f.count = hn[v].count; f.axis = 0; }
-            }
-        });
-        out->max_depth = (int)level_start.size() - 1;
+        out->order.resize(n);
+        GK(cudaMemcpyAsync(out->nodes.data(), D.flat, (size_t)nodes_used * sizeof(rtb::FlatNode), cudaMemcpyDeviceToHost, s));
+        GK(cudaMemcpyAsync(out->order.data(), D.perm, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, s));
+        GK(cudaStreamSynchronize(s));
+        GK(cudaGetLastError());
+        out->max_depth = levels;
     }
 done:
     cudaFree(arena);
