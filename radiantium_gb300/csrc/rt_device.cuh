@@ -854,37 +854,35 @@ DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status
 }
 
 /* The whole traversal of one ray by one thread. */
-template <HitForm kForm, bool kWide = false>
+template <HitForm kForm>
 DF void Traverse(const RtSceneView* S, const Ray& ray, Traversal& T, int2* stack, uint32_t* status, TravStats* st) {
-    if (TraversalBegin<kWide>(S, ray, T, st)) return;
+    if (TraversalBegin(S, ray, T, st)) return;
     const bool general = st || S->general_trees;
     while (true) {
         if (++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); return; }
         for (int k = 0; k < RT_DESCEND && T.cur >= 0; k++) {
-            if (kWide || general) {
-                if (DescendStep<int2*, kWide ? kNodesWide : kNodesGeneral>(T, stack, status, st)) return;
+            if (general) {
+                if (DescendStep<int2*, kNodesGeneral>(T, stack, status, st)) return;
             } else {
                 DescendStep<int2*, kNodesShort>(T, stack, status, nullptr);
             }
         }
-        if (T.cur < 0 && LeafStep<kForm, int2*, kWide>(S, T, stack, status, st)) return;
+        if (T.cur < 0 && LeafStep<kForm>(S, T, stack, status, st)) return;
     }
 }
 
 /* The closest hit of one ray; ray.MaxT ends at it. */
-template <bool kWide = false>
 DF bool SceneClosest(const RtSceneView* S, Ray& ray, Best* best, int2* stack, uint32_t* status, TravStats* st) {
     Traversal T;
-    Traverse<kClosestHit, kWide>(S, ray, T, stack, status, st);
+    Traverse<kClosestHit>(S, ray, T, stack, status, st);
     *best = T.best;
     ray.MaxT = T.inProto ? T.wMaxT : T.r.MaxT;
     return T.any;
 }
 
-template <bool kWide = false>
 DF bool SceneAny(const RtSceneView* S, const Ray& ray, int2* stack, uint32_t* status, TravStats* st) {
     Traversal T;
-    Traverse<kAnyHit, kWide>(S, ray, T, stack, status, st);
+    Traverse<kAnyHit>(S, ray, T, stack, status, st);
     return T.any;
 }
 

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(WF_FINISH_BLOCK, kKind == kFinishPath ? RT_FIN
             __syncwarp();
             int next = 0;
             if (count > 0)
-                trace_rays<kEitherHit, false, kMode>(W, RT_FINISH_REFILL, [&](unsigned idle, bool* exhausted) {
+                trace_queued<kEitherHit, false, kMode>(W, RT_FINISH_REFILL, [&](unsigned idle, bool* exhausted) {
                     const int e = next + __popc(idle & ((1u << lane) - 1u));
                     next += __popc(idle);
                     *exhausted = next >= count;

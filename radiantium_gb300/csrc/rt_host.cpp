@@ -99,6 +99,7 @@ struct Ctx {
     float* out = nullptr; size_t out_bytes = 0;
     unsigned char* noalloc = nullptr;          /* this device's fixed scratch (rt_noalloc.cu) */
     uint32_t* status = nullptr;
+    int32_t* next_ray = nullptr;               /* ray batches: the next ray to hand out */
     unsigned long long* stats = nullptr;
     void* io = nullptr; size_t io_bytes = 0;   /* device staging for host-pointer calls */
     bool counting = false;
@@ -1702,8 +1703,9 @@ void trace(Ctx* c, const rt_ray* rays, int64_t n, rt_hit* hits, uint8_t* occ, bo
         char* ob = base + (((size_t)n * sizeof(rt_ray) + 255) & ~(size_t)255);
         if (hits) dh = (rt_hit*)ob; else dob = (uint8_t*)ob;
     }
-    CK(rt_launch_trace(c->d_view, dr, n, dh, dob, c->status, c->stats, c->counting, s,
-                       c->traversal == RT_TRAVERSAL_WIDE && c->view.wide_ok));
+    CK(rt_launch_trace(c->d_view, dr, n, dh, dob, c->next_ray, c->status, c->stats, c->counting, s,
+                       c->tallest >= RT_DEEP_TREE, c->traversal == RT_TRAVERSAL_WIDE && c->view.wide_ok,
+                       c->view.general_trees != 0));
     if (host && n > 0) {
         if (hits) CK(cudaMemcpyAsync(hits, dh, (size_t)n * sizeof(rt_hit), cudaMemcpyDeviceToHost, s));
         else CK(cudaMemcpyAsync(occ, dob, (size_t)n, cudaMemcpyDeviceToHost, s));
@@ -1756,6 +1758,7 @@ int rt_create(int device, void** out_ctx) {
         CK(cudaEventCreateWithFlags(&c->fork.fork, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&c->fork.join, cudaEventDisableTiming));
         CK(rt_dev_malloc((void**)&c->status, 4));
+        CK(rt_dev_malloc((void**)&c->next_ray, 4));
         CK(rt_dev_malloc((void**)&c->stats, 8 * sizeof(unsigned long long)));
     });
     if (rc != RT_OK) { rt_destroy(c); return rc; }
@@ -1777,6 +1780,7 @@ void rt_destroy(void* ctx) {
     if (c->out) cudaFree(c->out);
     if (c->io) cudaFree(c->io);
     if (c->status) cudaFree(c->status);
+    if (c->next_ray) cudaFree(c->next_ray);
     if (c->stats) cudaFree(c->stats);
     free_wf(c);
     if (c->wf_exec) cudaGraphExecDestroy(c->wf_exec);

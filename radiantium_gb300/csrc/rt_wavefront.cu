@@ -74,7 +74,7 @@ template <bool kSh, NodeMode kMode>
 __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_CLOSEST_BLOCKS) k_wf_trace_closest(WfState W, uint32_t* status, unsigned long long* stats,
                                                             bool counting) {
     const int n = min(W.ctr->n_closest, 2 * W.slots);
-    trace_rays<kClosestHit, kSh, kMode>(W, W.refill, [&](unsigned idle, bool* exhausted) {
+    trace_queued<kClosestHit, kSh, kMode>(W, W.refill, [&](unsigned idle, bool* exhausted) {
         const int e = fetch_entry(&W.ctr->fetch[0], n, idle, exhausted);
         return e < n ? e : -1;
     }, status, stats, counting);
@@ -85,7 +85,7 @@ template <bool kSh, NodeMode kMode>
 __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_SHADOW_BLOCKS) k_wf_trace_shadow(WfState W, uint32_t* status, unsigned long long* stats,
                                                            bool counting) {
     const int n = min(W.ctr->n_shadow, 2 * W.slots);
-    trace_rays<kAnyHit, kSh, kMode>(W, W.refill, [&](unsigned idle, bool* exhausted) {
+    trace_queued<kAnyHit, kSh, kMode>(W, W.refill, [&](unsigned idle, bool* exhausted) {
         const int e = fetch_entry(&W.ctr->fetch[1], n, idle, exhausted);
         return e < n ? W.shadow_base + e : -1;
     }, status, stats, counting);

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include "rt_integrators.cuh"
 #include "rt_adjoint.cuh"
+#include "rt_trace.cuh"
 #include "rt_wavefront.h"
 
 using namespace rtd;
@@ -30,12 +31,6 @@ enum : uint32_t {
     F_ANY = 4096u,       /* the pending BSDF-sample term's ray is an any-hit ray (WF_RAY_MIS_ANY) */
     F_ALL = 2048u,       /* path, All light strategy: the vertex's lights are estimated one per iteration */
 };
-
-DF void warp_add64(unsigned long long* dst, uint32_t v) {
-    unsigned mask = __activemask();
-    uint32_t s = __reduce_add_sync(mask, v);
-    if ((threadIdx.x & 31) == (unsigned)(__ffs(mask) - 1) && s) atomicAdd(dst, (unsigned long long)s);
-}
 
 /* warp-aggregated append to a queue counter */
 DF int warp_append(int* counter, bool want) {
@@ -207,25 +202,6 @@ DF bool init_path(const WfState& W, int slot, long long sid, float4* o, float4* 
     return true;
 }
 
-/* Persistent traversal with dynamic ray fetch (Aila & Laine 2009): each warp
- * keeps its lanes busy by handing a new queue entry to every lane whose ray
- * has finished, as soon as W.refill lanes are idle, instead of idling until
- * the warp's longest ray is done.  The traversal is the step machine of
- * Traversal, so a lane can take a new ray between any two steps
- * and the per-ray results are the same as a one-ray-per-thread launch. */
-constexpr unsigned kFullWarp = 0xffffffffu;
-
-/* One warp-wide fetch: returns this lane's queue entry (>= n: none) and sets
- * `exhausted` (warp-uniform) once the queue has been handed out. */
-DF int fetch_entry(int32_t* counter, int n, unsigned idle, bool* exhausted) {
-    const unsigned lane = threadIdx.x & 31;
-    int first = 0;
-    if (lane == 0) first = atomicAdd(counter, __popc(idle));
-    first = __shfl_sync(kFullWarp, first, 0);
-    *exhausted = first + __popc(idle) >= n;
-    return first + __popc(idle & ((1u << lane) - 1u));
-}
-
 DF Ray queued_ray(const WfState& W, int q) {
     const float4 o = W.q_o[q], d = W.q_d[q];
     return mkray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, d.w);
@@ -239,23 +215,6 @@ DF void closest_done(const WfState& W, int meta, const Traversal& T) {
     else if (kind == WF_RAY_MIS) { W.mis_hit[path] = h; W.mis_sub[path] = T.best.sub; }
     else { W.trw_hit[path] = h; W.trw_sub[path] = T.best.sub; }
 }
-
-/* The traversal stack of a trace kernel: with kSh (scenes with tall trees)
- * its bottom RT_SH_STACK entries live in shared memory, which keeps the stack
- * of a deep traversal out of the L1 lines the node data needs; shallow trees
- * keep the whole stack in local memory, where it stays in a few hot lines. */
-template <bool kSh> struct TraceStack;
-template <> struct TraceStack<false> {
-    int2 a[2 * RT_STACK_SIZE];
-    DF int2* get() { return a; }
-};
-template <> struct TraceStack<true> {
-    int2 a[2 * RT_STACK_SIZE];
-    DF SplitStack get() {
-        __shared__ int2 sh[RT_SH_STACK * RT_TRACE_BLOCK];
-        return SplitStack{sh + threadIdx.x, a};
-    }
-};
 
 /* a shadow ray's answer: the path's occlusion flag, or for a light-tracer
  * camera connection its splat, added to the film sums when nothing is in the
@@ -274,90 +233,19 @@ DF void shadow_done(const WfState& W, int meta, bool hit) {
 }
 
 
-/* When a warp stops descending: as soon as this many of 32 live lanes wait for
- * a LeafStep (a share of the live lanes when fewer are live).  A low count
- * runs the leaf, instance-entry and instance-exit code for few lanes at a
- * time, a high one lets the lanes that reached a leaf idle; deep trees reach
- * leaves less often, so they wait less.  Trace ms of a 64-spp Cornell frame
- * (5-level tree) at 12 / 16 / 20 / 24: 3.70 / 3.58 / 3.53 / 3.52, against 3.73
- * with up to three nodes and one leaf per step; of a 16-spp pass over the
- * 64 x 200 k-triangle instances at 4 / 8 / 12 / 14 / 16 / 20: 82.7 / 76.3 /
- * 73.1 / 72.8 / 72.7 / 75.3, against 79.6 with up to five nodes per step. */
-#ifndef RT_LEAF_WAIT
-#define RT_LEAF_WAIT 22          /* shallow trees */
-#endif
-#ifndef RT_LEAF_WAIT_DEEP
-#define RT_LEAF_WAIT_DEEP 14     /* trees of RT_DEEP_TREE levels and more */
-#endif
-/* nodes a lane may visit in one run before the warp's fetch check (8 to 64 measured alike) */
-#ifndef RT_DESCEND_RUN
-#define RT_DESCEND_RUN 16
-#endif
-
-/* The traversal of a list of rays by one warp.  Lane by lane, `fetch` hands
- * out entries of W's ray arrays (-1: none for this lane; called by the whole
- * warp when at least `refill` lanes are idle, until it sets its second
- * argument); for kEitherHit the entry's top bit marks an any-hit ray.
- * Bound by lane utilisation and by the latency of dependent node loads (the
- * tree sits in L2): lanes at nodes, leaves and instance boundaries would
- * otherwise run one after another in every step, so the warp runs one kind at
- * a time for all lanes that wait for it. */
-#define WF_ANY_BIT ((int)0x80000000)
+/* The rays of W's queue: `fetch` hands out its entries (for kEitherHit an entry's
+ * top bit marks an any-hit ray), the results go to the paths' state. */
 template <HitForm kForm, bool kSh, NodeMode kMode, class Fetch>
-DF void trace_rays(const WfState& W, int refill, Fetch fetch, uint32_t* status, unsigned long long* stats, bool counting) {
-    constexpr bool kWide = kMode == kNodesWide;
-    if (kMode == kNodesShort) counting = false;
-    TraceStack<kSh> stk;
-    const auto stack = stk.get();
-    typedef decltype(stk.get()) Stk;
-    TravStats st = {0, 0, 0};
-    TravStats* pst = counting ? &st : nullptr;
-    uint32_t done = 0;
-    Traversal T;
-    T.cur = RT_NO_NODE;
-    T.first = kForm == kAnyHit;
-    const RtSceneView* S = nullptr;
+DF void trace_queued(const WfState& W, int refill, Fetch fetch, uint32_t* status, unsigned long long* stats, bool counting) {
     int meta = 0;
-    bool on = false, exhausted = false;      /* on: the lane has a ray */
-    auto finish = [&]() {
+    trace_rays<kForm, kSh, kMode>(refill, fetch, [&](int q, Ray* ray) {
+        meta = W.q_meta[q];
+        *ray = queued_ray(W, q);
+        return W.jobs[meta_job(meta)].view;
+    }, [&](const RtSceneView*, const Traversal& T) {
         if (kForm == kAnyHit || (kForm == kEitherHit && T.first)) shadow_done(W, meta, T.any);
         else closest_done(W, meta, T);
-        done++;
-        on = false;
-        T.cur = RT_NO_NODE;
-    };
-    while (true) {
-        const unsigned busy = __ballot_sync(kFullWarp, on);
-        if (exhausted) {
-            if (!busy) break;
-        } else if (32 - __popc(busy) >= refill) {
-            const int e = fetch(~busy, &exhausted);
-            if (!on && e != -1) {
-                const int q = kForm == kEitherHit ? e & ~WF_ANY_BIT : e;
-                if (kForm == kEitherHit) T.first = e < 0;
-                on = true;
-                meta = W.q_meta[q];
-                S = W.jobs[meta_job(meta)].view;
-                if (TraversalBegin<kWide>(S, queued_ray(W, q), T, pst)) finish();
-            }
-        }
-        bool over = false;
-        if (on && ++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); over = true; T.cur = RT_NO_NODE; }
-        const int live = __popc(__ballot_sync(kFullWarp, on && !over));
-        const int wait = (live * (kSh ? RT_LEAF_WAIT_DEEP : RT_LEAF_WAIT) + 31) >> 5;
-#pragma unroll 1
-        for (int k = 0; k < RT_DESCEND_RUN; k++) {
-            if (T.cur >= 0 && DescendStep<Stk, kMode>(T, stack, status, pst)) over = true;
-            if (live - __popc(__ballot_sync(kFullWarp, T.cur >= 0)) >= wait) break;
-        }
-        if (on && T.cur < 0 && (over || LeafStep<kForm, Stk, kWide>(S, T, stack, status, pst))) finish();
-    }
-    if (counting) {
-        warp_add64(stats + (kForm == kAnyHit ? 2 : 1), done);
-        warp_add64(stats + 3, st.nodes);
-        warp_add64(stats + 4, st.prims);
-        warp_add64(stats + 5, st.insts);
-    }
+    }, status, stats, counting);
 }
 
 DF bool load_hit(const RtSceneView* S, const Ray& ray, float4 h, int sub, Isect* it) {
@@ -1336,16 +1224,6 @@ DF bool shade_particle(const WfState& W, int slot, uint32_t* status, PartOut* o)
 }
 
 inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
-
-/* resident blocks of a grid-stride kernel: every SM filled once */
-template <typename K>
-int resident_blocks(K kernel, int block) {
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0) != cudaSuccess || per_sm <= 0)
-        per_sm = 1, sms = sms > 0 ? sms : 1;
-    return sms * per_sm;
-}
 
 }  // namespace
 
