@@ -98,11 +98,16 @@ struct Ctx {
     float* film = nullptr; size_t film_bytes = 0;
     float* out = nullptr; size_t out_bytes = 0;
     unsigned char* noalloc = nullptr;          /* this device's fixed scratch (rt_noalloc.cu) */
-    uint32_t* status = nullptr;
-    int32_t* next_ray = nullptr;               /* ray batches: the next ray to hand out */
-    unsigned long long* stats = nullptr;
+    /* the device words of a call, zeroed by one memset before it and read by one copy after it */
+    char* head = nullptr;
+    char* h_head = nullptr;                    /* pinned mirror */
+    uint32_t* status = nullptr;                /* head + 0 */
+    int32_t* next_ray = nullptr;               /* head + 64: ray batches, the next ray to hand out */
+    unsigned long long* stats = nullptr;       /* head + 128 */
     void* io = nullptr; size_t io_bytes = 0;   /* device staging for host-pointer calls */
     bool counting = false;
+    bool unfinished = false;                   /* a call has begun and not finished (begin_call) */
+    bool late_ms = false;                      /* events[0..1] hold the last round's time (finish_call) */
     rt_stats last{};
     uint64_t h2d = 0;                          /* host -> device bytes copied by the current call */
     std::atomic<int> cancel{0};
@@ -858,17 +863,37 @@ void throw_status(uint32_t st) {
     if (st & RT_STATUS_BOUNDS) throw RtFail(RT_ERR_BOUNDS, "a device index left its buffer (debug-bounds build)");
 }
 
-void check_status(Ctx* c) {
-    uint32_t st = 0;
-    CK(cudaMemcpyAsync(&st, c->status, 4, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+#define RT_HEAD_BYTES 192
+
+/* A call that ended early (a cancel, an error) may have left work queued that
+ * still reads the pinned staging: the next one waits for it first. */
+void begin_call(Ctx* c, cudaStream_t s) {
+    if (c->unfinished) CK(cudaDeviceSynchronize());
+    c->unfinished = true;
+    c->late_ms = false;
+    CK(cudaMemsetAsync(c->head, 0, RT_HEAD_BYTES, s));
+}
+
+/* ends a call's work on s: waits for it, reads the call's words and throws for
+ * a status; read_stats may follow */
+void finish_call(Ctx* c, cudaStream_t s) {
+    CK(cudaMemcpyAsync(c->h_head, c->head, RT_HEAD_BYTES, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    c->unfinished = false;
+    if (c->late_ms) {                          /* the last round's time, taken without a wait of its own */
+        float ms = 0;
+        CK(cudaEventElapsedTime(&ms, c->events[0], c->events[1]));
+        c->last.render_kernel_ms += ms;
+        c->late_ms = false;
+    }
+    uint32_t st;
+    std::memcpy(&st, c->h_head, 4);
     throw_status(st);
 }
 
 void read_stats(Ctx* c) {
     unsigned long long s[8];
-    CK(cudaMemcpyAsync(s, c->stats, sizeof(s), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    std::memcpy(s, c->h_head + 128, sizeof(s));
     c->last.rays_closest = s[1]; c->last.rays_shadow = s[2]; c->last.node_visits = s[3];
     c->last.prim_tests = s[4]; c->last.instance_visits = s[5]; c->last.invalid_samples = s[6];
 }
@@ -896,8 +921,7 @@ void render(Ctx* c, const rt_render_params* p, float* dst, bool dst_host, cudaSt
     ensure(&c->samples, &c->samples_bytes, (size_t)npix * chunk * 12);
     ensure(&c->film, &c->film_bytes, (size_t)npix * 12);
     CK(cudaMemsetAsync(c->film, 0, (size_t)npix * 12, s));
-    CK(cudaMemsetAsync(c->status, 0, 4, s));
-    CK(cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), s));
+    begin_call(c, s);
     c->cancel.store(0);
     /* the wavefront runs path with either light strategy, vol_path with Uniform */
     const bool wf_ok = P.strategy == RT_STRATEGY_UNIFORM || P.integrator == RT_INTEGRATOR_PATH;
@@ -916,8 +940,7 @@ void render(Ctx* c, const rt_render_params* p, float* dst, bool dst_host, cudaSt
     }
     CK(rt_launch_finalize(out, c->film, npix, (float)P.spp, s));
     if (dst_host) CK(cudaMemcpyAsync(dst, out, (size_t)npix * 12, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    check_status(c);
+    finish_call(c, s);
     double rms = c->last.render_kernel_ms, sms = c->last.shade_kernel_ms;
     uint64_t launches = c->last.kernel_launches, rl = c->last.render_launches;
     std::memset(&c->last, 0, sizeof(c->last));
@@ -997,6 +1020,7 @@ struct WfMode {
 struct WfTotals {
     double trace_ms = 0, shade_ms = 0;
     uint64_t launches = 0, trace_launches = 0;
+    bool late = false;       /* the last round is still running, its time in events[0..1] */
 };
 
 /* Active paths from which rt_wf_finish ends a round (measured, ms; off / 8 Ki /
@@ -1026,6 +1050,13 @@ int whole_round(const Ctx* c, const WfMode& m) {
  * with no more paths than finish_max has no loop. */
 void wf_round(Ctx* c, WfState W, cudaStream_t s, bool use_graph, const WfMode& m, int pass,
               const WfAdjoint* adj, int64_t total, int n_jobs, WfTotals* t) {
+    if (t->late) {                             /* the round before this one: its staging and events are needed again */
+        CK(cudaStreamSynchronize(s));
+        float ms = 0;
+        CK(cudaEventElapsedTime(&ms, c->events[0], c->events[1]));
+        t->trace_ms += ms;
+        t->late = false;
+    }
     W.finish_max = pass == WF_PASS_REPLAY || c->counting || m.general ? 0 : finish_at(c, m);
     std::memset(c->h_ctr, 0, sizeof(WfCounters));
     c->h_ctr->total = total;
@@ -1050,8 +1081,7 @@ void wf_round(Ctx* c, WfState W, cudaStream_t s, bool use_graph, const WfMode& m
     if (W.finish_max > 0 && std::min<int64_t>(W.slots, total) <= whole_round(c, m)) {
         if (c->cancel.load()) throw RtFail(RT_ERR_CANCELLED, "render cancelled");
         end_round();
-        CK(cudaStreamSynchronize(s));
-        add_ms(0, &t->trace_ms);
+        t->late = true;
         return;
     }
     if (use_graph && pass == WF_PASS_RENDER) {
@@ -1090,8 +1120,7 @@ void wf_round(Ctx* c, WfState W, cudaStream_t s, bool use_graph, const WfMode& m
     }
     if (active() > 0 || c->h_ctr->n_shadow > 0) {
         end_round();
-        CK(cudaStreamSynchronize(s));
-        add_ms(0, &t->trace_ms);
+        t->late = true;
     }
 }
 
@@ -1100,6 +1129,7 @@ void wf_store_totals(Ctx* c, const WfTotals& t) {
     c->last.shade_kernel_ms = t.shade_ms;
     c->last.render_launches = t.trace_launches;
     c->last.kernel_launches = t.launches;
+    c->late_ms = t.late;
 }
 
 /* The light tracer as a wavefront (rt_wavefront.cu): rounds of up to
@@ -1131,7 +1161,7 @@ void particle_wavefront(Ctx* c, const RtParams& P, int64_t first, int64_t count,
     for (int64_t done = 0; done < count;) {
         if (c->cancel.load()) throw RtFail(RT_ERR_CANCELLED, "render cancelled");
         const int64_t n = std::min(round_max, count - done);
-        CK(cudaStreamSynchronize(s));          /* the pinned staging is free */
+        if (done > 0) CK(cudaStreamSynchronize(s));   /* the pinned staging of the last round has been read */
         WfJob& d = c->h_jobs[0];
         d.view = c->d_view;
         d.P = P;
@@ -1157,8 +1187,7 @@ void render_particles(Ctx* c, const rt_render_params* p, int64_t first, int64_t 
     ensure(&c->film, &c->film_bytes, (size_t)npix * 16);    /* float4 sums: one vector atomic per splat */
     float4* film = reinterpret_cast<float4*>(c->film);
     CK(cudaMemsetAsync(film, 0, (size_t)npix * 16, s));
-    CK(cudaMemsetAsync(c->status, 0, 4, s));
-    CK(cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), s));
+    begin_call(c, s);
     c->cancel.store(0);
     const bool mega = c->renderer == RT_RENDERER_MEGAKERNEL;
     const int64_t chunk = std::max<int64_t>(1, c->sample_budget);
@@ -1181,7 +1210,6 @@ void render_particles(Ctx* c, const rt_render_params* p, int64_t first, int64_t 
         particle_wavefront(c, P, first, count, c->film, s,
                            c->renderer == RT_RENDERER_WAVEFRONT_GRAPH || c->renderer == RT_RENDERER_AUTO);
     }
-    const rt_stats wf_last = c->last;
     float* out = dst;
     if (dst_host) {
         ensure(&c->out, &c->out_bytes, (size_t)npix * 12);
@@ -1191,8 +1219,8 @@ void render_particles(Ctx* c, const rt_render_params* p, int64_t first, int64_t 
     const float v = (float)P.w * (float)P.h / (float)count;
     CK(rt_launch_particle_finish(c->d_view, npix, film, v, out, c->status, c->stats, c->counting, s));
     if (dst_host) CK(cudaMemcpyAsync(dst, out, (size_t)npix * 12, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    check_status(c);
+    finish_call(c, s);
+    const rt_stats wf_last = c->last;
     double ms = 0;
     for (int64_t ci = 0; ci < nchunks; ci++) {
         float t = 0;
@@ -1228,15 +1256,14 @@ void particle_splats(Ctx* c, const rt_render_params* p, int64_t first, int64_t c
     int32_t* dn = (int32_t*)buf;
     int32_t* dp = (int32_t*)(buf + nb);
     float* dr = (float*)(buf + nb + pb);
-    CK(cudaMemsetAsync(c->status, 0, 4, c->stream));
+    begin_call(c, c->stream);
     CK(rt_launch_particle_records(c->d_view, P, first, count, dn, dp, dr, max_per, c->status, c->stream));
     CK(cudaMemcpyAsync(n, dn, nb, cudaMemcpyDeviceToHost, c->stream));
     if (max_per > 0) {
         CK(cudaMemcpyAsync(pix, dp, pb, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaMemcpyAsync(rgb, dr, rb, cudaMemcpyDeviceToHost, c->stream));
     }
-    CK(cudaStreamSynchronize(c->stream));
-    check_status(c);
+    finish_call(c, c->stream);
 }
 
 /* rt_render_device_noalloc: the megakernel render with every buffer carved
@@ -1387,6 +1414,7 @@ void wavefront_run(Ctx* c, const std::vector<WfJobIn>& jobs, cudaStream_t s, boo
     for (const WfJobIn& J : jobs) mode.general = mode.general || J.general;
     ensure_events(c, 4);
     WfTotals tot;
+    bool first_round = true;
     while (true) {
         if (c->cancel.load()) throw RtFail(RT_ERR_CANCELLED, "render cancelled");
         std::vector<int> act;
@@ -1405,7 +1433,8 @@ void wavefront_run(Ctx* c, const std::vector<WfJobIn>& jobs, cudaStream_t s, boo
         ensure(&c->samples, &c->samples_bytes, (size_t)total * 12);
         const int slots = (int)std::min<int64_t>(std::min<int64_t>(c->wf_capacity, WF_MAX_SLOTS), total + 31);
         ensure_wf(c, slots);
-        CK(cudaStreamSynchronize(s));          /* the pinned staging of the last round has been read */
+        if (!first_round) CK(cudaStreamSynchronize(s));   /* the pinned staging of the last round has been read */
+        first_round = false;
         int64_t first = 0;
         for (size_t k = 0; k < act.size(); k++) {
             const WfJobIn& J = jobs[act[k]];
@@ -1509,8 +1538,7 @@ void render_batch(Ctx* c, const rt_batch_item* items, int n, bool device_out, cu
     if (!device_out) ensure(&c->out, &c->out_bytes, (size_t)film_floats * 4);
     for (int i = 0; i < n; i++) jobs[i].film = c->film + film_off[i];
     CK(cudaMemsetAsync(c->film, 0, (size_t)film_floats * 4, s));
-    CK(cudaMemsetAsync(c->status, 0, 4, s));
-    CK(cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), s));
+    begin_call(c, s);
     c->cancel.store(0);
     wavefront_run(c, jobs, s, c->renderer == RT_RENDERER_WAVEFRONT_GRAPH ||
                               (c->renderer == RT_RENDERER_AUTO && c->wf_graph_pref));
@@ -1525,8 +1553,7 @@ void render_batch(Ctx* c, const rt_batch_item* items, int n, bool device_out, cu
         }
         samples += (uint64_t)npix * jobs[i].P.spp;
     }
-    CK(cudaStreamSynchronize(s));
-    check_status(c);
+    finish_call(c, s);
     double rms = c->last.render_kernel_ms, sms = c->last.shade_kernel_ms;
     uint64_t launches = c->last.kernel_launches, rl = c->last.render_launches;
     std::memset(&c->last, 0, sizeof(c->last));
@@ -1585,7 +1612,7 @@ void adjoint_backward(Ctx* c, const rt_render_params* p, const rt_adjoint_desc* 
     CK(rt_launch_scale(c->adj_dldi, npix * 3, 1.0f / (float)P.spp, s));
     CK(cudaMemsetAsync(c->adj_galb, 0, (size_t)std::max<int64_t>(1, texels) * 12, s));
     CK(cudaMemsetAsync(c->adj_galpha, 0, (size_t)std::max(1, d->alpha_count) * 4, s));
-    CK(cudaMemsetAsync(c->status, 0, 4, s));
+    begin_call(c, s);
     c->cancel.store(0);
     const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(P.spp, c->sample_budget / std::max<int64_t>(1, npix)));
     ensure_events(c, 4);
@@ -1605,7 +1632,6 @@ void adjoint_backward(Ctx* c, const rt_render_params* p, const rt_adjoint_desc* 
         jobs[0].tallest = c->tallest;
         jobs[0].wide_ok = c->view.wide_ok != 0;
     jobs[0].general = c->view.general_trees != 0;
-        CK(cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), s));
         wavefront_run(c, jobs, s, false, &A);
         launches += c->last.kernel_launches;
     } else {
@@ -1621,8 +1647,7 @@ void adjoint_backward(Ctx* c, const rt_render_params* p, const rt_adjoint_desc* 
     CK(cudaEventRecord(e1, s));
     if (texels > 0) CK(cudaMemcpyAsync(g_albedo, c->adj_galb, (size_t)texels * 12, cudaMemcpyDeviceToHost, s));
     if (d->alpha_count > 0) CK(cudaMemcpyAsync(g_alpha, c->adj_galpha, (size_t)d->alpha_count * 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    check_status(c);
+    finish_call(c, s);
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
@@ -1689,8 +1714,7 @@ void trace(Ctx* c, const rt_ray* rays, int64_t n, rt_hit* hits, uint8_t* occ, bo
     if (!c->has_scene) throw RtFail(RT_ERR_NO_SCENE, "no scene uploaded");
     if (n < 0 || (n > 0 && (!rays || (!hits && !occ)))) throw RtFail(RT_ERR_INVALID_ARG, "trace: bad arguments");
     cudaStream_t s = user ? user : c->stream;
-    CK(cudaMemsetAsync(c->status, 0, 4, s));
-    CK(cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), s));
+    begin_call(c, s);
     const rt_ray* dr = rays;
     rt_hit* dh = hits;
     uint8_t* dob = occ;
@@ -1710,8 +1734,7 @@ void trace(Ctx* c, const rt_ray* rays, int64_t n, rt_hit* hits, uint8_t* occ, bo
         if (hits) CK(cudaMemcpyAsync(hits, dh, (size_t)n * sizeof(rt_hit), cudaMemcpyDeviceToHost, s));
         else CK(cudaMemcpyAsync(occ, dob, (size_t)n, cudaMemcpyDeviceToHost, s));
     }
-    CK(cudaStreamSynchronize(s));
-    check_status(c);
+    finish_call(c, s);
     std::memset(&c->last, 0, sizeof(c->last));
     c->last.h2d_bytes = c->h2d;
     read_stats(c);
@@ -1757,9 +1780,11 @@ int rt_create(int device, void** out_ctx) {
         CK(cudaStreamCreateWithFlags(&c->fork.side, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&c->fork.fork, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&c->fork.join, cudaEventDisableTiming));
-        CK(rt_dev_malloc((void**)&c->status, 4));
-        CK(rt_dev_malloc((void**)&c->next_ray, 4));
-        CK(rt_dev_malloc((void**)&c->stats, 8 * sizeof(unsigned long long)));
+        CK(rt_dev_malloc((void**)&c->head, RT_HEAD_BYTES));
+        CK(cudaMallocHost((void**)&c->h_head, RT_HEAD_BYTES));
+        c->status = (uint32_t*)c->head;
+        c->next_ray = (int32_t*)(c->head + 64);
+        c->stats = (unsigned long long*)(c->head + 128);
     });
     if (rc != RT_OK) { rt_destroy(c); return rc; }
     *out_ctx = c;
@@ -1779,9 +1804,8 @@ void rt_destroy(void* ctx) {
     if (c->adj_slot) cudaFree(c->adj_slot);
     if (c->out) cudaFree(c->out);
     if (c->io) cudaFree(c->io);
-    if (c->status) cudaFree(c->status);
-    if (c->next_ray) cudaFree(c->next_ray);
-    if (c->stats) cudaFree(c->stats);
+    if (c->head) cudaFree(c->head);
+    if (c->h_head) cudaFreeHost(c->h_head);
     free_wf(c);
     if (c->wf_exec) cudaGraphExecDestroy(c->wf_exec);
     if (c->wf_graph) cudaGraphDestroy(c->wf_graph);

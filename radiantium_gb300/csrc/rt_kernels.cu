@@ -213,7 +213,7 @@ cudaError_t rt_launch_trace(const RtSceneView* S, const rt_ray* rays, int64_t n,
     const int64_t most = 1 << 30;              /* ray indices are 32-bit in the kernel */
     for (int64_t first = 0; first < n; first += most) {
         const int len = (int)std::min(most, n - first);
-        cudaError_t e = cudaMemsetAsync(next, 0, sizeof(int32_t), stream);
+        cudaError_t e = first > 0 ? cudaMemsetAsync(next, 0, sizeof(int32_t), stream) : cudaSuccess;
         if (e != cudaSuccess) return e;
         const unsigned g = std::min<unsigned>(grid_for(len, RT_TRACE_BLOCK), (unsigned)grids.blocks[a][m][d]);
         kBatch[a][m][d]<<<g, RT_TRACE_BLOCK, 0, stream>>>(S, rays + first, len, hits ? hits + first : nullptr,

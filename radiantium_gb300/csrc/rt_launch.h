@@ -14,7 +14,7 @@ cudaError_t rt_launch_render(const RtSceneView* S, const RtParams& P, float* sam
 cudaError_t rt_launch_accumulate(float* film, const float* samples, int64_t npix, int chunk_len, cudaStream_t stream);
 cudaError_t rt_launch_finalize(float* out, const float* film, int64_t npix, float spp, cudaStream_t stream);
 /* a ray batch, closest hits (hits) or any hits (occ); `next`: a device counter
- * for handing out rays; deep, wide, general: as rt_wf_trace's */
+ * for handing out rays, 0 at the call; deep, wide, general: as rt_wf_trace's */
 cudaError_t rt_launch_trace(const RtSceneView* S, const rt_ray* rays, int64_t n, rt_hit* hits, uint8_t* occ,
                             int32_t* next, uint32_t* status, unsigned long long* stats, bool counting, cudaStream_t stream,
                             bool deep, bool wide, bool general);

@@ -34,8 +34,12 @@ template <class T> using Array = std::vector<T, NoInit<T>>;
 template <class F>
 void parallel_for(int64_t n, int64_t grain, F&& f) {
     if (n <= 0) return;
-    const int64_t cores = std::max(1u, std::thread::hardware_concurrency());
-    const int64_t parts = std::min(cores, std::max<int64_t>(1, n / std::max<int64_t>(1, grain)));
+    static const int64_t cores = std::max(1u, std::thread::hardware_concurrency());   /* it reads /sys */
+    const int64_t parts = std::min(cores, n / std::max<int64_t>(1, grain));
+    if (parts <= 1) {
+        f((int64_t)0, n);
+        return;
+    }
     std::exception_ptr failed;
     std::mutex lock;
     auto range = [&](int64_t k) {
