@@ -86,6 +86,13 @@ DF V3 XfN12(V3 v, const float* m) {
               v.x * m[1] + v.y * m[4] + v.z * m[7],
               v.x * m[2] + v.y * m[5] + v.z * m[8]);
 }
+/* the 12 floats of a matrix in read-only global memory, 16-byte aligned */
+DF void load12(const float4* p, float (&m)[12]) {
+    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+    m[0] = a.x; m[1] = a.y; m[2] = a.z; m[3] = a.w;
+    m[4] = b.x; m[5] = b.y; m[6] = b.z; m[7] = b.w;
+    m[8] = c.x; m[9] = c.y; m[10] = c.z; m[11] = c.w;
+}
 /* full Matrix4x4 (16 floats, M11..M44) used by the camera */
 DF V3 Xf16(V3 p, const float* m) {
     return v3(p.x * m[0] + p.y * m[4] + p.z * m[8] + m[12],
@@ -456,12 +463,11 @@ DF bool PrimHit(const RtSceneView* S, uint32_t kind, uint32_t ref, float4 s0, fl
     return SphereTest(v3(sph.center[0], sph.center[1], sph.center[2]), sph.radius, r, t);
 }
 
-/* Root box of tree `bvh`: RT_NO_NODE if the tree is empty or the box is
+/* Root box of tree `h`: RT_NO_NODE if the tree is empty or the box is
  * missed, else the root's reference (counts one node visit if non-empty);
  * kWide: the root of the tree's wide form. */
 template <bool kWide = false>
-DF int RootRef(const RtSceneView* S, int bvh, const Ray& r, TravStats* st) {
-    const RtBvh h = S->bvhs[bvh];
+DF int RootRef(const RtBvh& h, const Ray& r, TravStats* st) {
     if (h.root_ref == RT_NO_NODE) return RT_NO_NODE;
     if (st) st->nodes++;
     float tmin;
@@ -715,7 +721,7 @@ DF bool TraversalBegin(const RtSceneView* S, const Ray& ray, Traversal& T, TravS
     T.pt = kFMax; T.pu = 0; T.pv = 0; T.pslot = -1; T.pflags = 0;
     T.guard = 0;
     T.nodes = kWide ? S->wnodes : S->nodes;
-    T.cur = RootRef<kWide>(S, 0, ray, st);
+    T.cur = RootRef<kWide>(S->top, ray, st);
     return T.cur == RT_NO_NODE;
 }
 
@@ -801,15 +807,16 @@ DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status
         T.inst = (int)ref;
         T.topSlot = T.leafSlot; T.topLeft = T.leafLeft; T.leafLeft = 0;
         T.wMaxT = T.r.MaxT;
-        const RtInstance& I = S->instances[T.inst];
+        const float4* I = reinterpret_cast<const float4*>(S->instances + T.inst);
         float w2m[12];
-#pragma unroll
-        for (int i = 0; i < 12; i++) w2m[i] = __ldg(I.w2m + i);
+        load12(I, w2m);
+        const float4 h0 = __ldg(I + 3), h1 = __ldg(I + 4);
         T.r = XfRay(T.r, w2m);
         T.pt = kFMax; T.pu = 0; T.pv = 0; T.pslot = -1; T.pflags = 0; T.pany = false;
         T.inProto = true;
         T.base = T.sp;
-        T.cur = RootRef<kWide>(S, 1 + __ldg(&I.blas), T.r, st);
+        const RtBvh root = {{h0.x, h0.y, h0.z}, {h0.w, h1.x, h1.y}, __float_as_int(h1.z), __float_as_int(h1.w)};
+        T.cur = RootRef<kWide>(root, T.r, st);
         return false;
     }
     if (!T.inProto) return true;
@@ -831,8 +838,7 @@ DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status
             pm = n * sph.radius + c;
         }
         float m2w[12];
-#pragma unroll
-        for (int i = 0; i < 12; i++) m2w[i] = __ldg(I.m2w + i);
+        load12(reinterpret_cast<const float4*>(I.m2w), m2w);
         const V3 pw = Xf12(pm, m2w);
         const float t = Distance(T.wO, pw);
         T.any = true;
@@ -908,6 +914,7 @@ DF void Finish(const RtSceneView* S, const Ray& ray, const Best& b, Isect* it) {
     } else {
         const RtInstance& I = S->instances[ref];
         float w2m[12], m2w[12];
+        /* plain loads: as vectors the matrices cost every shade registers (Cornell frame 7.40 -> 7.61 ms) */
         for (int i = 0; i < 12; i++) { w2m[i] = I.w2m[i]; m2w[i] = I.m2w[i]; }
         V3 dm = Normalize(XfN12(ray.D, w2m));
         float4 p0 = __ldg(S->slots + 3 * (int64_t)b.sub);

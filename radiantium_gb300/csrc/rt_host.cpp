@@ -676,7 +676,7 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
             check_index(gd.ref, d->blas_count, "instanced prototype");
             RtInstance I{};
             rows12(gd.model_to_world, I.m2w); rows12(gd.world_to_model, I.w2m);
-            I.blas = gd.ref;
+            I.root = bvhs[1 + gd.ref];
             int id = (int)prims.size();
             prims.push_back(RtPrim{RT_KIND_INSTANCE, (int)insts.size(), tp.material, -1, tp.med_in, tp.med_out, 0, 0});
             boxes.push_back(xform_box(blas_root[gd.ref], gd.model_to_world));
@@ -786,7 +786,7 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
     RtSceneView& v = c->view;
     v.nodes = upload(c, nodes);
     v.slots = upload(c, slots);
-    v.bvhs = upload(c, bvhs);
+    v.top = bvhs[0];
     v.prims = upload(c, prims);
     v.tris = upload(c, tris);
     v.pos = upload(c, pos);
