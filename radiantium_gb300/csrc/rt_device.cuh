@@ -860,14 +860,15 @@ DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status
 }
 
 /* The whole traversal of one ray by one thread (the megakernels).  Bound by
- * divergence: nothing gathers a warp's lanes here, and with both forms of the
- * node visit in one loop they drift apart (Cornell frame 127 ms, 49 before the
- * forms were split), so each form has its own loop.  The short form descends
- * until the ray is at a leaf; ms with the megakernels at 3 / 5 / 16 / 64 nodes a
- * turn: Cornell frame 37.2 / 32.9 / 31.7 / 31.6, volume 104 / 92 / 86 / 83, light
- * tracer 108 / 80 / 74 / 74, 8-spp pass over the 64 instances 376 / 341 / 311 / 298.
- * The general form, which counts in registers, visits one node a turn: counting
- * Cornell frame 70, at three nodes 118. */
+ * latency at a few warps an SM and by divergence.  Each form of the node visit
+ * has a loop of its own: with both in one loop, chosen per node, a Cornell
+ * frame took 127 ms, with the split 37.  The short form descends until the ray
+ * is at a leaf; ms with the megakernels at 3 / 5 / 16 / 64 nodes a turn: Cornell
+ * frame 37.2 / 32.9 / 31.7 / 31.6, volume 104 / 92 / 86 / 83, light tracer 108 / 80 /
+ * 74 / 74, 8-spp pass over the 64 instances 376 / 341 / 311 / 298.  The general
+ * form, which counts in registers, visits one node a turn: counting Cornell
+ * frame 70, at three nodes 118.  Bringing the warp's lanes together each turn,
+ * as the persistent kernels do, is slower in both: 58 and 147. */
 template <HitForm kForm>
 DF void Traverse(const RtSceneView* S, const Ray& ray, Traversal& T, int2* stack, uint32_t* status, TravStats* st) {
     if (TraversalBegin(S, ray, T, st)) return;
