@@ -544,15 +544,21 @@ DF int VisitNode(const float4* nodes, int node, const Ray& r, Stk stack, int* sp
  * fmaxf / fminf ignore it), one on x fails the box (x0 <= x1 fails).  Both
  * children's plane distances are computed as packed pairs - the node stores
  * left and right planes side by side - with (plane - o) as plane + (-o), the
- * same bits.  A far child that fails its test, or lies beyond MaxT already
- * (which only shrinks), would be popped and dropped, so it is not pushed; one
- * whose sibling missed is visited next without a trip through the stack.
+ * same bits.  A far child that fails its test would be popped and dropped, so
+ * it is not pushed, nor is one that lies beyond MaxT already where MaxT only
+ * shrinks (kNodesShort); one whose sibling missed is visited next without a
+ * trip through the stack.
+ * kGrow: `grow` tells that MaxT may still grow.  It does at one place: leaving
+ * a prototype sets it to the world distance of the ray's first hit, which can
+ * exceed the finite MaxT that the ray came with (a direction longer than 1, or
+ * rounding).  A far child beyond MaxT may then pass when it is popped, so it
+ * is pushed too.
  * Bound by instruction issue and dependent node loads, not by bytes: against
  * the general form, trace ms of a 16-spp pass over the 64 x 200 k-triangle
  * instances 72.8 -> 55.3, of a 64-spp Cornell frame 3.52 -> 2.58; 2 M
  * incoherent rays 2.41 -> 1.98 ms. */
-template <class Stk>
-DF int VisitNodeFast(const float4* nodes, int node, const Ray& r, Stk stack, int* sp, int base) {
+template <bool kGrow, class Stk>
+DF int VisitNodeFast(const float4* nodes, int node, const Ray& r, bool grow, Stk stack, int* sp, int base) {
     f32x2 a[4], b[4];                    /* min x, max x, min y, max y; min z, max z, refs, axis */
     ldg32(nodes + 4 * (int64_t)node, a);
     ldg32(nodes + 4 * (int64_t)node + 2, b);
@@ -564,15 +570,19 @@ DF int VisitNodeFast(const float4* nodes, int node, const Ray& r, Stk stack, int
     const f32x2 z0 = mul2(add2(nz ? b[1] : b[0], oz), iz), z1 = mul2(add2(nz ? b[0] : b[1], oz), iz);
     const float tl = fmaxf(fmaxf(lo2(x0), lo2(y0)), lo2(z0)), el = fminf(fminf(lo2(x1), lo2(y1)), lo2(z1));
     const float tr = fmaxf(fmaxf(hi2(x0), hi2(y0)), hi2(z0)), er = fminf(fminf(hi2(x1), hi2(y1)), hi2(z1));
-    const bool hl = (lo2(x0) <= lo2(x1)) & (tl <= el) & (el > 0.0f) & (tl < r.MaxT);
-    const bool hr = (hi2(x0) <= hi2(x1)) & (tr <= er) & (er > 0.0f) & (tr < r.MaxT);
+    const bool bl = (lo2(x0) <= lo2(x1)) & (tl <= el) & (el > 0.0f), br = (hi2(x0) <= hi2(x1)) & (tr <= er) & (er > 0.0f);
+    const bool hl = bl & (tl < r.MaxT), hr = br & (tr < r.MaxT);
     const int lref = (int)(uint32_t)b[2], rref = (int)(uint32_t)(b[2] >> 32), axis = (int)(uint32_t)b[3];
     if (hl & hr) {
         const bool rightFirst = axis == 0 ? nx : (axis == 1 ? ny : nz);
         stk_put(stack, (*sp)++, make_int2(rightFirst ? lref : rref, __float_as_int(rightFirst ? tl : tr)));
         return rightFirst ? rref : lref;
     }
-    if (hl | hr) return hl ? lref : rref;
+    if (hl | hr) {
+        if (kGrow && grow && (hl ? br : bl) && hl == !(axis == 0 ? nx : (axis == 1 ? ny : nz)))
+            stk_put(stack, (*sp)++, make_int2(hl ? rref : lref, __float_as_int(hl ? tr : tl)));    /* the far one, beyond MaxT */
+        return hl ? lref : rref;
+    }
     return PopNext(stack, sp, base, r.MaxT, nullptr);
 }
 
@@ -726,16 +736,24 @@ DF bool TraversalBegin(const RtSceneView* S, const Ray& ray, Traversal& T, TravS
 }
 
 /* How a traversal visits nodes: in the general form (node counts, any tree),
- * in the short form (no counts, trees that cannot overflow the stack), or the
- * fast traversal's wide nodes (a visit may push up to seven entries). */
-enum NodeMode { kNodesGeneral, kNodesShort, kNodesWide };
+ * in the short form (no counts, trees that cannot overflow the stack), in the
+ * fast traversal's wide nodes (a visit may push up to seven entries), or in
+ * the short form for closest-hit rays whose MaxT may grow (VisitNodeFast's
+ * kGrow).  That takes a scene with instances and a finite MaxT that a hit can
+ * exceed: a ray batch's, that of vol_path's walks to a light, and the camera's
+ * far plane where it does not lie behind the whole scene (RtSceneView::far_cuts).
+ * The others keep the plain short form, because the test costs every visit:
+ * 16-spp pass over the 64 instances 67.6 -> 68.2 ms, Cornell frame 7.42 -> 7.53,
+ * 256 x 256 preview 0.36 -> 0.38; 2 M incoherent rays, which have it, 1.31 -> 1.32. */
+enum NodeMode { kNodesGeneral, kNodesShort, kNodesWide, kNodesGrow };
 
 /* One interior node (T.cur >= 0).  Returns true when the traversal has
  * finished (a top-level stack overflow). */
 template <class Stk, NodeMode kMode>
 DF bool DescendStep(Traversal& T, Stk stack, uint32_t* status, TravStats* st) {
-    if (kMode == kNodesShort) {
-        T.cur = VisitNodeFast(T.nodes, T.cur, T.r, stack, &T.sp, T.base);
+    if (kMode == kNodesShort || kMode == kNodesGrow) {
+        const bool grow = T.best.t == kFMax && T.r.MaxT < kFMax;     /* no hit yet, and a finite MaxT */
+        T.cur = VisitNodeFast<kMode == kNodesGrow>(T.nodes, T.cur, T.r, grow, stack, &T.sp, T.base);
         return false;
     }
     if (kMode == kNodesWide ? T.sp - T.base > RT_STACK_SIZE - 8 : T.sp - T.base == RT_STACK_SIZE) {
@@ -884,7 +902,7 @@ DF void Traverse(const RtSceneView* S, const Ray& ray, Traversal& T, int2* stack
     }
     while (true) {
         if (++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); return; }
-        for (int k = 0; k < RT_DESCEND && T.cur >= 0; k++) DescendStep<int2*, kNodesShort>(T, stack, status, nullptr);
+        for (int k = 0; k < RT_DESCEND && T.cur >= 0; k++) DescendStep<int2*, kForm == kAnyHit ? kNodesShort : kNodesGrow>(T, stack, status, nullptr);
         if (T.cur < 0 && LeafStep<kForm>(S, T, stack, status, nullptr)) return;
     }
 }

@@ -138,28 +138,29 @@ __global__ void __launch_bounds__(WF_FINISH_BLOCK, kKind == kFinishPath ? RT_FIN
 }
 
 typedef void (*FinishKernel)(WfState, uint32_t*, unsigned long long*, int);
-/* by [kind][wide nodes] */
-const FinishKernel kFinish[3][2] = {
-    {k_wf_finish<kFinishPath, kNodesShort>, k_wf_finish<kFinishPath, kNodesWide>},
-    {k_wf_finish<kFinishVol, kNodesShort>, k_wf_finish<kFinishVol, kNodesWide>},
-    {k_wf_finish<kFinishParticle, kNodesShort>, k_wf_finish<kFinishParticle, kNodesWide>}};
+/* by [kind][short, wide, grow]; the light tracer's closest-hit rays have no finite MaxT */
+const FinishKernel kFinish[3][3] = {
+    {k_wf_finish<kFinishPath, kNodesShort>, k_wf_finish<kFinishPath, kNodesWide>, k_wf_finish<kFinishPath, kNodesGrow>},
+    {k_wf_finish<kFinishVol, kNodesShort>, k_wf_finish<kFinishVol, kNodesWide>, k_wf_finish<kFinishVol, kNodesGrow>},
+    {k_wf_finish<kFinishParticle, kNodesShort>, k_wf_finish<kFinishParticle, kNodesWide>,
+     k_wf_finish<kFinishParticle, kNodesShort>}};
 
 struct FinishGrids {
-    int blocks[3][2];
+    int blocks[3][3];
     FinishGrids() {
         for (int k = 0; k < 3; k++)
-            for (int w = 0; w < 2; w++) blocks[k][w] = resident_blocks(kFinish[k][w], WF_FINISH_BLOCK);
+            for (int w = 0; w < 3; w++) blocks[k][w] = resident_blocks(kFinish[k][w], WF_FINISH_BLOCK);
     }
 };
 
 }  // namespace
 
 cudaError_t rt_wf_finish(const WfState& W, uint32_t* status, unsigned long long* stats, cudaStream_t s, int pass, bool vol,
-                         bool particle, bool wide) {
+                         bool particle, bool wide, bool grow) {
     static const FinishGrids grids;
     cudaError_t e = rt_wf_phase(W, s);
     if (e != cudaSuccess) return e;
-    const int k = particle ? kFinishParticle : (vol ? kFinishVol : kFinishPath), w = wide ? 1 : 0;
+    const int k = particle ? kFinishParticle : (vol ? kFinishVol : kFinishPath), w = wide ? 1 : (grow ? 2 : 0);
     kFinish[k][w]<<<grids.blocks[k][w], WF_FINISH_BLOCK, 0, s>>>(W, status, stats, pass);
     return cudaGetLastError();
 }

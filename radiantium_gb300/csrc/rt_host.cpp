@@ -617,6 +617,7 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
     std::vector<RtLight> lights;
     std::vector<int32_t> infinite;
     std::vector<RtInstance> insts;
+    float inst_terms = 0;                      /* largest sum of the terms of an instance's point, by size */
     auto area_light = [&](int kind, int ref, const rt_group_desc& gd, float area) {
         RtLight L{};
         L.kind = kind; L.ref = ref; L.le[0] = gd.le[0]; L.le[1] = gd.le[1]; L.le[2] = gd.le[2]; L.area = area;
@@ -677,6 +678,12 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
             RtInstance I{};
             rows12(gd.model_to_world, I.m2w); rows12(gd.world_to_model, I.w2m);
             I.root = bvhs[1 + gd.ref];
+            for (int j = 0; j < 3; j++) {
+                float terms = std::fabs(gd.model_to_world[12 + j]);
+                for (int k = 0; k < 3; k++)
+                    terms += std::fabs(gd.model_to_world[4 * k + j]) * std::max(std::fabs(I.root.root_min[k]), std::fabs(I.root.root_max[k]));
+                inst_terms = std::max(inst_terms, terms);
+            }
             int id = (int)prims.size();
             prims.push_back(RtPrim{RT_KIND_INSTANCE, (int)insts.size(), tp.material, -1, tp.med_in, tp.med_out, 0, 0});
             boxes.push_back(xform_box(blas_root[gd.ref], gd.model_to_world));
@@ -818,6 +825,7 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
     v.global_medium = d->global_medium < 0 ? -1 : d->global_medium;
     const bool overflows = tallest > RT_STACK_SIZE + 1;
     v.general_trees = overflows || odd_boxes ? 1 : 0;
+    v.instanced = insts.empty() ? 0 : 1;
     c->tallest = tallest;
     if (wnodes.empty()) wnodes.push_back(make_float4(0, 0, 0, 0));
     v.wnodes = upload(c, wnodes);
@@ -845,6 +853,18 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
         cam.max_x = pmin[0]; cam.max_y = pmin[1];
         const float area = std::fabs((cam.max_x - cam.min_x) * (cam.max_y - cam.min_y));
         cam.normalization = 1 / area;
+    }
+    /* an instance's hit point lies in the top-level box, which holds its transformed
+     * prototype, so none is further from the camera than the box's farthest corner; the
+     * rounding of the points (of their terms' size) and of the distance is covered amply */
+    {
+        float corner[3];
+        for (int k = 0; k < 3; k++) {
+            const float at = cam.camera_to_world[12 + k];
+            corner[k] = std::max(std::fabs(v.top.root_min[k] - at), std::fabs(v.top.root_max[k] - at));
+        }
+        const float reach = length(f3(corner[0], corner[1], corner[2])) + 1e-5f * inst_terms;
+        v.far_cuts = reach < 0.999f * cam.far_z ? 0 : 1;
     }
     c->d_view = upload(c, std::vector<RtSceneView>{v});
     CK(cudaStreamSynchronize(c->stream));
@@ -1014,6 +1034,7 @@ struct WfMode {
     bool deep = false;       /* trace kernels with the shared-memory stack (trees of 16+ levels) */
     bool wide = false;       /* the opt-in fast traversal over the wide nodes */
     bool general = false;    /* a scene's trees need the general node visit */
+    bool grow = false;       /* closest-hit rays whose MaxT may grow (kNodesGrow) */
     bool one_type = false;   /* one scene, one material type */
 };
 /* CUDA-event times and launch counts of a run, summed over its rounds */
@@ -1072,8 +1093,8 @@ void wf_round(Ctx* c, WfState W, cudaStream_t s, bool use_graph, const WfMode& m
     /* the rays of the paths that are left, then the paths to their end; stream order, no wait */
     auto end_round = [&]() {
         CK(cudaEventRecord(c->events[0], s));
-        CK(rt_wf_trace(W, c->status, c->stats, c->counting, s, m.deep, m.wide, m.general, &c->fork));
-        CK(rt_wf_finish(W, c->status, c->stats, s, pass, m.vol, m.particle, m.wide));
+        CK(rt_wf_trace(W, c->status, c->stats, c->counting, s, m.deep, m.wide, m.general, m.grow, &c->fork));
+        CK(rt_wf_finish(W, c->status, c->stats, s, pass, m.vol, m.particle, m.wide, m.grow));
         CK(cudaEventRecord(c->events[1], s));
         t->launches += 4;
         t->trace_launches += 2;
@@ -1105,7 +1126,7 @@ void wf_round(Ctx* c, WfState W, cudaStream_t s, bool use_graph, const WfMode& m
         if (c->h_ctr->iter >= W.iter_cap) throw RtFail(RT_ERR_ITER_CAP, "wavefront: bounce iteration cap reached (WF_ITER_CAP)");
         NvtxRange nvtx_iter("rt.wavefront_iteration");
         CK(cudaEventRecord(c->events[0], s));
-        CK(rt_wf_trace(W, c->status, c->stats, c->counting, s, m.deep, m.wide, m.general, &c->fork));
+        CK(rt_wf_trace(W, c->status, c->stats, c->counting, s, m.deep, m.wide, m.general, m.grow, &c->fork));
         CK(cudaEventRecord(c->events[1], s));
         CK(cudaEventRecord(c->events[2], s));
         CK(rt_wf_shade(W, active(), c->status, c->stats, c->counting, 0, false, s, &t->launches, pass, adj, m.vol,
@@ -1339,6 +1360,8 @@ struct WfJobIn {
     int tallest;           /* levels of its tallest tree */
     bool wide_ok;          /* its wide trees fit the fast traversal's stack */
     bool general;          /* its trees need the general node visit */
+    bool instanced;        /* it has instances */
+    bool far_cuts;         /* its camera's far plane may lie before a hit */
 };
 
 /* The bounce loop as a graph: a while node whose body is one iteration
@@ -1346,7 +1369,7 @@ struct WfJobIn {
  * condition when no path is left.  Rebuilt when the path state moves or the
  * counting mode changes. */
 void ensure_wf_graph(Ctx* c, const WfState& W, const WfMode& m) {
-    const uint64_t key = (c->wf_generation << 32) ^ ((uint64_t)m.wide << 63) ^ ((uint64_t)m.general << 62) ^ ((uint64_t)W.slots << 10) ^ ((uint64_t)m.deep << 9) ^
+    const uint64_t key = (c->wf_generation << 32) ^ ((uint64_t)m.wide << 63) ^ ((uint64_t)m.general << 62) ^ ((uint64_t)m.grow << 61) ^ ((uint64_t)W.slots << 10) ^ ((uint64_t)m.deep << 9) ^
                          ((uint64_t)(uint32_t)W.iter_cap * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)(uint32_t)W.finish_max * 0xC2B2AE3D27D4EB4Full) ^
                          ((uint64_t)m.sort << 8) ^ ((uint64_t)m.particle << 7) ^ ((uint64_t)W.refill << 2) ^
                          ((uint64_t)m.vol << 1) ^ (c->counting ? 1u : 0u);
@@ -1366,7 +1389,7 @@ void ensure_wf_graph(Ctx* c, const WfState& W, const WfMode& m) {
     cudaGraph_t body = np.conditional.phGraph_out[0];
     CK(cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     uint64_t launches = 0;
-    cudaError_t e1 = rt_wf_trace(W, c->status, c->stats, c->counting, c->stream, m.deep, m.wide, m.general, &c->fork);
+    cudaError_t e1 = rt_wf_trace(W, c->status, c->stats, c->counting, c->stream, m.deep, m.wide, m.general, m.grow, &c->fork);
     cudaError_t e2 = rt_wf_shade(W, -1, c->status, c->stats, c->counting, loop, true, c->stream, &launches,
                                  WF_PASS_RENDER, nullptr, m.vol, m.particle, m.sort);
     cudaGraph_t captured = nullptr;
@@ -1375,8 +1398,8 @@ void ensure_wf_graph(Ctx* c, const WfState& W, const WfMode& m) {
     CK(e2);
     if (W.finish_max > 0) {                    /* after the loop: the paths that are left */
         CK(cudaStreamBeginCaptureToGraph(c->stream, c->wf_graph, &node, nullptr, 1, cudaStreamCaptureModeRelaxed));
-        e1 = rt_wf_trace(W, c->status, c->stats, c->counting, c->stream, m.deep, m.wide, m.general, &c->fork);
-        e2 = rt_wf_finish(W, c->status, c->stats, c->stream, WF_PASS_RENDER, m.vol, m.particle, m.wide);
+        e1 = rt_wf_trace(W, c->status, c->stats, c->counting, c->stream, m.deep, m.wide, m.general, m.grow, &c->fork);
+        e2 = rt_wf_finish(W, c->status, c->stats, c->stream, WF_PASS_RENDER, m.vol, m.particle, m.wide, m.grow);
         CK(cudaStreamEndCapture(c->stream, &captured));
         CK(e1);
         CK(e2);
@@ -1412,6 +1435,7 @@ void wavefront_run(Ctx* c, const std::vector<WfJobIn>& jobs, cudaStream_t s, boo
     mode.wide = c->traversal == RT_TRAVERSAL_WIDE;
     for (const WfJobIn& J : jobs) mode.wide = mode.wide && J.wide_ok;
     for (const WfJobIn& J : jobs) mode.general = mode.general || J.general;
+    for (const WfJobIn& J : jobs) mode.grow = mode.grow || (J.instanced && (vol || J.far_cuts));
     ensure_events(c, 4);
     WfTotals tot;
     bool first_round = true;
@@ -1488,6 +1512,8 @@ void render_wavefront(Ctx* c, RtParams P, int chunk, int64_t npix, cudaStream_t 
     jobs[0].tallest = c->tallest;
     jobs[0].wide_ok = c->view.wide_ok != 0;
     jobs[0].general = c->view.general_trees != 0;
+    jobs[0].instanced = c->view.instanced != 0;
+    jobs[0].far_cuts = c->view.far_cuts != 0;
     /* AUTO drives vol_path's loop as a graph: its boundary walks make ~100 short iterations per
      * round, where the host loop's per-iteration synchronisation costs 9 % (C3) */
     const bool vol = P.integrator == RT_INTEGRATOR_VOL_PATH;
@@ -1530,6 +1556,8 @@ void render_batch(Ctx* c, const rt_batch_item* items, int n, bool device_out, cu
         jobs[i].tallest = sc->tallest;
         jobs[i].wide_ok = sc->view.wide_ok != 0;
         jobs[i].general = sc->view.general_trees != 0;
+        jobs[i].instanced = sc->view.instanced != 0;
+        jobs[i].far_cuts = sc->view.far_cuts != 0;
         film_off[i] = film_floats;
         film_floats += (int64_t)P.w * P.h * 3;
     }
@@ -1632,6 +1660,8 @@ void adjoint_backward(Ctx* c, const rt_render_params* p, const rt_adjoint_desc* 
         jobs[0].tallest = c->tallest;
         jobs[0].wide_ok = c->view.wide_ok != 0;
     jobs[0].general = c->view.general_trees != 0;
+    jobs[0].instanced = c->view.instanced != 0;
+    jobs[0].far_cuts = c->view.far_cuts != 0;
         wavefront_run(c, jobs, s, false, &A);
         launches += c->last.kernel_launches;
     } else {
@@ -1729,7 +1759,7 @@ void trace(Ctx* c, const rt_ray* rays, int64_t n, rt_hit* hits, uint8_t* occ, bo
     }
     CK(rt_launch_trace(c->d_view, dr, n, dh, dob, c->next_ray, c->status, c->stats, c->counting, s,
                        c->tallest >= RT_DEEP_TREE, c->traversal == RT_TRAVERSAL_WIDE && c->view.wide_ok,
-                       c->view.general_trees != 0));
+                       c->view.general_trees != 0, c->view.instanced != 0));
     if (host && n > 0) {
         if (hits) CK(cudaMemcpyAsync(hits, dh, (size_t)n * sizeof(rt_hit), cudaMemcpyDeviceToHost, s));
         else CK(cudaMemcpyAsync(occ, dob, (size_t)n, cudaMemcpyDeviceToHost, s));

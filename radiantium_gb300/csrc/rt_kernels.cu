@@ -185,20 +185,22 @@ namespace {
 
 typedef void (*BatchKernel)(const RtSceneView*, const rt_ray*, int, rt_hit*, uint8_t*, int32_t*, uint32_t*,
                             unsigned long long*, bool);
-/* by [any-hit][node mode][shared-memory stack] */
-const BatchKernel kBatch[2][3][2] = {
+/* by [any-hit][node mode][shared-memory stack] (any-hit rays never change MaxT) */
+const BatchKernel kBatch[2][4][2] = {
     {{k_trace<false, false, kNodesGeneral>, k_trace<false, true, kNodesGeneral>},
      {k_trace<false, false, kNodesShort>, k_trace<false, true, kNodesShort>},
-     {k_trace<false, false, kNodesWide>, k_trace<false, true, kNodesWide>}},
+     {k_trace<false, false, kNodesWide>, k_trace<false, true, kNodesWide>},
+     {k_trace<false, false, kNodesGrow>, k_trace<false, true, kNodesGrow>}},
     {{k_trace<true, false, kNodesGeneral>, k_trace<true, true, kNodesGeneral>},
      {k_trace<true, false, kNodesShort>, k_trace<true, true, kNodesShort>},
-     {k_trace<true, false, kNodesWide>, k_trace<true, true, kNodesWide>}}};
+     {k_trace<true, false, kNodesWide>, k_trace<true, true, kNodesWide>},
+     {k_trace<true, false, kNodesShort>, k_trace<true, true, kNodesShort>}}};
 
 struct BatchGrids {
-    int blocks[2][3][2];
+    int blocks[2][4][2];
     BatchGrids() {
         for (int a = 0; a < 2; a++)
-            for (int m = 0; m < 3; m++)
+            for (int m = 0; m < 4; m++)
                 for (int d = 0; d < 2; d++) blocks[a][m][d] = resident_blocks(kBatch[a][m][d], RT_TRACE_BLOCK);
     }
 };
@@ -207,9 +209,9 @@ struct BatchGrids {
 
 cudaError_t rt_launch_trace(const RtSceneView* S, const rt_ray* rays, int64_t n, rt_hit* hits, uint8_t* occ,
                             int32_t* next, uint32_t* status, unsigned long long* stats, bool counting, cudaStream_t stream,
-                            bool deep, bool wide, bool general) {
+                            bool deep, bool wide, bool general, bool instanced) {
     static const BatchGrids grids;
-    const int a = hits ? 0 : 1, m = wide ? kNodesWide : (general || counting ? kNodesGeneral : kNodesShort), d = deep ? 1 : 0;
+    const int a = hits ? 0 : 1, m = wide ? kNodesWide : (general || counting ? kNodesGeneral : (instanced ? kNodesGrow : kNodesShort)), d = deep ? 1 : 0;
     const int64_t most = 1 << 30;              /* ray indices are 32-bit in the kernel */
     for (int64_t first = 0; first < n; first += most) {
         const int len = (int)std::min(most, n - first);

@@ -87,7 +87,7 @@ template <HitForm kForm, bool kSh, NodeMode kMode, class Fetch, class Load, clas
 DF void trace_rays(int refill, Fetch fetch, Load load, Report report, uint32_t* status, unsigned long long* stats,
                    bool counting) {
     constexpr bool kWide = kMode == kNodesWide;
-    if (kMode == kNodesShort) counting = false;
+    if (kMode == kNodesShort || kMode == kNodesGrow) counting = false;
     TraceStack<kSh> stk;
     const auto stack = stk.get();
     typedef decltype(stk.get()) Stk;

@@ -347,20 +347,22 @@ namespace {
 
 typedef void (*TraceKernel)(WfState, uint32_t*, unsigned long long*, bool);
 /* the trace kernels by [node mode][shared-memory stack] */
-const TraceKernel kClosest[3][2] = {
+const TraceKernel kClosest[4][2] = {
     {k_wf_trace_closest<false, kNodesGeneral>, k_wf_trace_closest<true, kNodesGeneral>},
     {k_wf_trace_closest<false, kNodesShort>, k_wf_trace_closest<true, kNodesShort>},
-    {k_wf_trace_closest<false, kNodesWide>, k_wf_trace_closest<true, kNodesWide>}};
-const TraceKernel kShadow[3][2] = {
+    {k_wf_trace_closest<false, kNodesWide>, k_wf_trace_closest<true, kNodesWide>},
+    {k_wf_trace_closest<false, kNodesGrow>, k_wf_trace_closest<true, kNodesGrow>}};
+const TraceKernel kShadow[4][2] = {
     {k_wf_trace_shadow<false, kNodesGeneral>, k_wf_trace_shadow<true, kNodesGeneral>},
     {k_wf_trace_shadow<false, kNodesShort>, k_wf_trace_shadow<true, kNodesShort>},
-    {k_wf_trace_shadow<false, kNodesWide>, k_wf_trace_shadow<true, kNodesWide>}};
+    {k_wf_trace_shadow<false, kNodesWide>, k_wf_trace_shadow<true, kNodesWide>},
+    {k_wf_trace_shadow<false, kNodesShort>, k_wf_trace_shadow<true, kNodesShort>}};
 
 /* resident blocks of every trace kernel */
 struct TraceGrids {
-    int closest[3][2], shadow[3][2];
+    int closest[4][2], shadow[4][2];
     TraceGrids() {
-        for (int m = 0; m < 3; m++)
+        for (int m = 0; m < 4; m++)
             for (int d = 0; d < 2; d++) {
                 closest[m][d] = resident_blocks(kClosest[m][d], RT_TRACE_BLOCK);
                 shadow[m][d] = resident_blocks(kShadow[m][d], RT_TRACE_BLOCK);
@@ -371,9 +373,9 @@ struct TraceGrids {
 }  // namespace
 
 cudaError_t rt_wf_trace(const WfState& W, uint32_t* status, unsigned long long* stats, bool counting, cudaStream_t s,
-                        bool deep, bool wide, bool general, const WfFork* fork) {
+                        bool deep, bool wide, bool general, bool grow, const WfFork* fork) {
     static const TraceGrids grids;
-    const int m = wide ? kNodesWide : (general || counting ? kNodesGeneral : kNodesShort), d = deep ? 1 : 0;
+    const int m = wide ? kNodesWide : (general || counting ? kNodesGeneral : (grow ? kNodesGrow : kNodesShort)), d = deep ? 1 : 0;
     cudaError_t e = cudaSuccess;
     if (fork) {
         e = cudaEventRecord(fork->fork, s);

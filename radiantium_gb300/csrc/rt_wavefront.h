@@ -135,7 +135,8 @@ cudaError_t rt_wf_start(const WfState& W, cudaStream_t s, bool particle = false)
  * `deep`: a tree of the scene has RT_DEEP_TREE levels or more, the kernels
  * keep the bottom of the traversal stack in shared memory.  `wide`: the
  * opt-in fast traversal over the scenes' wide nodes.  `general`: a scene has
- * RtSceneView::general_trees (counting runs use the general form too). */
+ * RtSceneView::general_trees (counting runs use the general form too).  `grow`:
+ * closest-hit rays whose MaxT may grow may be queued (kNodesGrow). */
 #ifndef RT_DEEP_TREE
 #define RT_DEEP_TREE 16
 #endif
@@ -148,7 +149,8 @@ struct WfFork {
     cudaEvent_t fork, join;
 };
 cudaError_t rt_wf_trace(const WfState& W, uint32_t* status, unsigned long long* stats, bool counting, cudaStream_t s,
-                        bool deep = false, bool wide = false, bool general = false, const WfFork* fork = nullptr);
+                        bool deep = false, bool wide = false, bool general = false, bool grow = false,
+                        const WfFork* fork = nullptr);
 /* Shades the active paths (`particle`: light-tracer particles) - regrouped by
  * shade key first with `sort` - then advances the iteration; with `loop` set
  * (inside a captured while-loop), also sets the loop's condition to "paths
@@ -165,6 +167,6 @@ cudaError_t rt_wf_phase(const WfState& W, cudaStream_t s);
  * path, whose rays have been traced, to its end (rt_finish.cu).  Not for the
  * adjoint's replay, for counting or for scenes with general_trees. */
 cudaError_t rt_wf_finish(const WfState& W, uint32_t* status, unsigned long long* stats, cudaStream_t s, int pass,
-                         bool vol, bool particle, bool wide);
+                         bool vol, bool particle, bool wide, bool grow);
 
 #endif
