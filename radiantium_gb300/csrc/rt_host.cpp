@@ -106,6 +106,7 @@ struct Ctx {
     unsigned long long* stats = nullptr;       /* head + 128 */
     void* io = nullptr; size_t io_bytes = 0;   /* device staging for host-pointer calls */
     bool counting = false;
+    cudaStream_t call_stream = nullptr;        /* the stream of the call that has begun */
     bool unfinished = false;                   /* a call has begun and not finished (begin_call) */
     bool late_ms = false;                      /* events[0..1] hold the last round's time (finish_call) */
     rt_stats last{};
@@ -885,13 +886,23 @@ void throw_status(uint32_t st) {
 
 #define RT_HEAD_BYTES 192
 
-/* A call that ended early (a cancel, an error) may have left work queued that
- * still reads the pinned staging: the next one waits for it first. */
+/* The first device work of a call on s. */
 void begin_call(Ctx* c, cudaStream_t s) {
-    if (c->unfinished) CK(cudaDeviceSynchronize());
+    c->call_stream = s;
     c->unfinished = true;
     c->late_ms = false;
     CK(cudaMemsetAsync(c->head, 0, RT_HEAD_BYTES, s));
+}
+
+/* A call that ends early (a cancel, an error) may leave a round queued on its
+ * stream, which still reads the pinned staging and the scenes and adds to the
+ * film: it returns when that is done, because the next call may clear the film
+ * from another stream, or upload another scene. */
+void drain_call(Ctx* c) {
+    if (!c->unfinished) return;
+    c->unfinished = false;
+    cudaStreamSynchronize(c->call_stream);
+    cudaStreamSynchronize(c->fork.side);
 }
 
 /* ends a call's work on s: waits for it, reads the call's words and throws for
@@ -938,10 +949,10 @@ void render(Ctx* c, const rt_render_params* p, float* dst, bool dst_host, cudaSt
     cudaStream_t s = user ? user : c->stream;
     const int64_t npix = (int64_t)P.w * P.h;
     int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(P.spp, c->sample_budget / std::max<int64_t>(1, npix)));
+    begin_call(c, s);
     ensure(&c->samples, &c->samples_bytes, (size_t)npix * chunk * 12);
     ensure(&c->film, &c->film_bytes, (size_t)npix * 12);
     CK(cudaMemsetAsync(c->film, 0, (size_t)npix * 12, s));
-    begin_call(c, s);
     c->cancel.store(0);
     /* the wavefront runs path with either light strategy, vol_path with Uniform */
     const bool wf_ok = P.strategy == RT_STRATEGY_UNIFORM || P.integrator == RT_INTEGRATOR_PATH;
@@ -1205,10 +1216,10 @@ void render_particles(Ctx* c, const rt_render_params* p, int64_t first, int64_t 
     if (!dst) throw RtFail(RT_ERR_INVALID_ARG, "render_particles: null output");
     cudaStream_t s = user ? user : c->stream;
     const int64_t npix = (int64_t)P.w * P.h;
+    begin_call(c, s);
     ensure(&c->film, &c->film_bytes, (size_t)npix * 16);    /* float4 sums: one vector atomic per splat */
     float4* film = reinterpret_cast<float4*>(c->film);
     CK(cudaMemsetAsync(film, 0, (size_t)npix * 16, s));
-    begin_call(c, s);
     c->cancel.store(0);
     const bool mega = c->renderer == RT_RENDERER_MEGAKERNEL;
     const int64_t chunk = std::max<int64_t>(1, c->sample_budget);
@@ -1562,11 +1573,11 @@ void render_batch(Ctx* c, const rt_batch_item* items, int n, bool device_out, cu
         film_floats += (int64_t)P.w * P.h * 3;
     }
     cudaStream_t s = device_out && user ? user : c->stream;
+    begin_call(c, s);
     ensure(&c->film, &c->film_bytes, (size_t)film_floats * 4);
     if (!device_out) ensure(&c->out, &c->out_bytes, (size_t)film_floats * 4);
     for (int i = 0; i < n; i++) jobs[i].film = c->film + film_off[i];
     CK(cudaMemsetAsync(c->film, 0, (size_t)film_floats * 4, s));
-    begin_call(c, s);
     c->cancel.store(0);
     wavefront_run(c, jobs, s, c->renderer == RT_RENDERER_WAVEFRONT_GRAPH ||
                               (c->renderer == RT_RENDERER_AUTO && c->wf_graph_pref));
@@ -1631,6 +1642,7 @@ void adjoint_backward(Ctx* c, const rt_render_params* p, const rt_adjoint_desc* 
     const int64_t npix = (int64_t)P.w * P.h;
     const int64_t texels = d->albedo_texture >= 0
         ? (int64_t)c->h_textures[d->albedo_texture].width * c->h_textures[d->albedo_texture].height : 0;
+    begin_call(c, s);
     ensure(&c->adj_dldi, &c->adj_dldi_bytes, (size_t)npix * 12);
     ensure(&c->adj_galb, &c->adj_galb_bytes, (size_t)std::max<int64_t>(1, texels) * 12);
     ensure(&c->adj_galpha, &c->adj_galpha_bytes, (size_t)std::max(1, d->alpha_count) * 4);
@@ -1640,7 +1652,6 @@ void adjoint_backward(Ctx* c, const rt_render_params* p, const rt_adjoint_desc* 
     CK(rt_launch_scale(c->adj_dldi, npix * 3, 1.0f / (float)P.spp, s));
     CK(cudaMemsetAsync(c->adj_galb, 0, (size_t)std::max<int64_t>(1, texels) * 12, s));
     CK(cudaMemsetAsync(c->adj_galpha, 0, (size_t)std::max(1, d->alpha_count) * 4, s));
-    begin_call(c, s);
     c->cancel.store(0);
     const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(P.spp, c->sample_budget / std::max<int64_t>(1, npix)));
     ensure_events(c, 4);
@@ -1782,12 +1793,15 @@ int run(Ctx* c, F f) {
         c->err.clear();
         return RT_OK;
     } catch (const RtFail& e) {
+        drain_call(c);
         c->err = e.what();
         return e.code;
     } catch (const std::bad_alloc&) {
+        drain_call(c);
         c->err = "host allocation failed";
         return RT_ERR_OOM;
     } catch (const std::exception& e) {
+        drain_call(c);
         c->err = e.what();
         return RT_ERR_INVALID_ARG;
     }
