@@ -10,7 +10,6 @@
 #include <memory>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -55,7 +54,7 @@ void parallel_for(int64_t n, int64_t grain, F&& f) {
     int64_t k = 1;
     try {
         for (; k < parts; k++) threads.emplace_back(range, k);
-    } catch (const std::system_error&) {
+    } catch (...) {                            /* no thread, or no memory for its state: the rest runs here */
     }
     range(0);
     for (; k < parts; k++) range(k);
