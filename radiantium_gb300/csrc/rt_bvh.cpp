@@ -201,7 +201,7 @@ BuildResult build_sah(const Array<Box>& prim_bounds, int max_prims, int threads)
 
 /* ---- the wide tree of the fast traversal -------------------------------------------------- */
 
-/* floor and ceil of log2(x), x > 0, and 2^k (-1022 <= k <= 1023) */
+/* floor and ceil of log2(x), x > 0 (any number for an infinite x), and 2^k (-1022 <= k <= 1023) */
 static int floor_log2(double x) {
     int e;
     std::frexp(x, &e);
@@ -235,10 +235,10 @@ static void quantise_axis(double mn, double mx, const Box* kids, int n, int axis
         float pf = (float)(mn - s);
         if ((double)pf > mn - s) pf = std::nextafter(pf, -INFINITY);
         bool ok = std::isfinite(pf);
-        int lo[8] = {0}, hi[8] = {0};
+        double lo[8], hi[8];                     /* not integers yet: an infinite box fits no grid */
         for (int c = 0; ok && c < n; c++) {
-            lo[c] = (int)std::floor(((double)kids[c].mn[axis] - (double)pf) / s) - 1;
-            hi[c] = (int)std::ceil(((double)kids[c].mx[axis] - (double)pf) / s) + 1;
+            lo[c] = std::floor(((double)kids[c].mn[axis] - (double)pf) / s) - 1;
+            hi[c] = std::ceil(((double)kids[c].mx[axis] - (double)pf) / s) + 1;
             ok = lo[c] >= 0 && hi[c] <= 255;
         }
         if (!ok) continue;
