@@ -441,9 +441,13 @@ struct Best {
 #ifndef RT_TRAVERSAL_CAP
 #define RT_TRAVERSAL_CAP (1u << 26)   /* loop steps of one two-level traversal */
 #endif
+/* interior nodes a thread that traverses a ray alone visits between two
+ * LeafSteps, in the short and the general form (Traverse) */
 #ifndef RT_DESCEND
-/* interior nodes a thread that traverses a ray alone visits between two LeafSteps */
 #define RT_DESCEND 64
+#endif
+#ifndef RT_DESCEND_GENERAL
+#define RT_DESCEND_GENERAL 6
 #endif
 #define RT_NO_NODE ((int)0x80000000)
 
@@ -877,32 +881,52 @@ DF bool LeafStep(const RtSceneView* S, Traversal& T, Stk stack, uint32_t* status
     return false;
 }
 
+/* One turn of a ray that one thread traverses alone, in the general form: up to
+ * RT_DESCEND_GENERAL nodes, then a LeafStep if they reached one.  True when the
+ * traversal has finished.  The same steps as DescendStep, with the overflow's
+ * returns inside the run: the lanes of a warp then run apart, which hides the
+ * latency of their loads (counting Cornell frame 50 ms; 141 with DescendStep
+ * called here, after which the compiler brings the lanes together). */
+template <HitForm kForm>
+DF bool GeneralTurn(const RtSceneView* S, Traversal& T, int2* stack, uint32_t* status, TravStats* st) {
+    if (++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); return true; }
+    if (T.cur != RT_NO_NODE) {
+        for (int k = 0; k < RT_DESCEND_GENERAL && T.cur >= 0; k++) {
+            if (T.sp - T.base == RT_STACK_SIZE) {
+                atomicOr(status, RT_STATUS_STACK);
+                if (!T.inProto) return true;
+                T.sp = T.base;                  /* the prototype's traversal stops here */
+                T.cur = RT_NO_NODE;
+                return false;
+            }
+            T.cur = VisitNode(T.nodes, T.cur, T.r, stack, &T.sp, T.base, st);
+        }
+        if (T.cur >= 0) return false;
+    }
+    return LeafStep<kForm>(S, T, stack, status, st);
+}
+
 /* The whole traversal of one ray by one thread (the megakernels).  Bound by
  * latency at a few warps an SM and by divergence.  Each form of the node visit
  * has a loop of its own: with both in one loop, chosen per node, a Cornell
- * frame took 127 ms, with the split 37.  The short form descends until the ray
- * is at a leaf; ms with the megakernels at 3 / 5 / 16 / 64 nodes a turn: Cornell
- * frame 37.2 / 32.9 / 31.7 / 31.6, volume 104 / 92 / 86 / 83, light tracer 108 / 80 /
- * 74 / 74, 8-spp pass over the 64 instances 376 / 341 / 311 / 298.  The general
- * form, which counts in registers, visits one node a turn: counting Cornell
- * frame 70, at three nodes 118.  Bringing the warp's lanes together each turn,
- * as the persistent kernels do, is slower in both: 58 and 147. */
+ * frame took 127 ms.  The short form descends until the ray is at a leaf; ms
+ * with the megakernels at 3 / 5 / 16 / 64 nodes a turn: Cornell frame 37.2 /
+ * 32.9 / 31.7 / 31.6, volume 104 / 92 / 86 / 83, light tracer 108 / 80 / 74 / 74,
+ * 8-spp pass over the 64 instances 376 / 341 / 311 / 298.  The general form,
+ * counting, at 2 / 3 / 4 / 6 nodes a turn: 55 / 50 / 47 / 43, 152 / 135 / 126 / 116,
+ * 216 / 163 / 144 / 120, 477 / 439 / 418 / 389.  Bringing the warp's lanes together each turn, as the
+ * persistent kernels do, is slower in both: Cornell frame 58 and 147. */
 template <HitForm kForm>
 DF void Traverse(const RtSceneView* S, const Ray& ray, Traversal& T, int2* stack, uint32_t* status, TravStats* st) {
     if (TraversalBegin(S, ray, T, st)) return;
     if (st || S->general_trees) {
-        TravStats n = {0, 0, 0};
-        while (true) {
-            if (++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); break; }
-            if (T.cur >= 0 && DescendStep<int2*, kNodesGeneral>(T, stack, status, &n)) break;
-            if (T.cur < 0 && LeafStep<kForm>(S, T, stack, status, &n)) break;
-        }
-        if (st) { st->nodes += n.nodes; st->prims += n.prims; st->insts += n.insts; }
+        while (!GeneralTurn<kForm>(S, T, stack, status, st)) {}
         return;
     }
     while (true) {
         if (++T.guard > RT_TRAVERSAL_CAP) { atomicOr(status, RT_STATUS_TRAV); return; }
-        for (int k = 0; k < RT_DESCEND && T.cur >= 0; k++) DescendStep<int2*, kForm == kAnyHit ? kNodesShort : kNodesGrow>(T, stack, status, nullptr);
+        for (int k = 0; k < RT_DESCEND && T.cur >= 0; k++)
+            DescendStep<int2*, kForm == kAnyHit ? kNodesShort : kNodesGrow>(T, stack, status, nullptr);
         if (T.cur < 0 && LeafStep<kForm>(S, T, stack, status, nullptr)) return;
     }
 }
