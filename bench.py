@@ -188,6 +188,21 @@ def cpu_baseline(scene, st, target_s, threads=0, frame_nodes_per_sample=None):
             "sample_nodes_per_sample": work, "frame_nodes_per_sample": frame_nodes_per_sample}
 
 
+def counting_passes(dev, render):
+    """One render counting the reference's rays and box tests, one counting those of the rays that a
+    run without counting traces: an infinite light's MIS ray stops at its first hit, and is traced
+    only where it carries a term.  Returns both sets of counts."""
+    out = []
+    dev.set_counting(True)
+    for traced in (False, True):
+        dev.count_traced(traced)
+        render()
+        out.append(dev.stats())
+    dev.count_traced(False)
+    dev.set_counting(False)
+    return out
+
+
 class ClockSampler:
     """nvidia-smi sampling during the timed region (every 200 ms)."""
 
@@ -369,12 +384,10 @@ def run_ours(args):
     graph_loop = mode == N.RENDERER_WAVEFRONT_GRAPH or (mode == N.RENDERER_AUTO and (
         st.integrator == N.INTEGRATOR_VOL_PATH or (tuned is not None and tuned["renderer"] == N.RENDERER_WAVEFRONT_GRAPH)))
 
-    # one untimed counting pass: exact traversal counts of this workload
-    dev.set_counting(True)
-    dev.render_device(st.replace(spp=spp_step, sample_begin=base), film.data_ptr(), stream)
-    torch.cuda.synchronize()
-    counts = dev.stats()
-    dev.set_counting(False)
+    # untimed counting passes of this workload: the reference's traversal counts (for the CPU
+    # sample), and those of the rays that the timed steps trace (rays/s and algorithmic bytes)
+    ref_counts, counts = counting_passes(dev, lambda: dev.render_device(
+        st.replace(spp=spp_step, sample_begin=base), film.data_ptr(), stream))
 
     dev.set_traversal(traversal)            # the counting pass above ran the exact traversal
     dev.set_light_sampling(light_sampling)
@@ -481,7 +494,7 @@ def run_ours(args):
         plain = {"value": samples_step / (float(np.mean(pt)) / 1000.0), "unit": "samples/s", "steps": args.plain_steps,
                  "note": "plain megakernel (one thread per camera sample), same passes, identical films"}
 
-    # roofline of the path-tracing kernel (algorithmic bytes from exact counts); a
+    # roofline of the path-tracing kernel (algorithmic bytes from the counts of the rays traced); a
     # graph-driven loop is timed as a whole, so the trace kernels' own time then
     # comes from one more (untimed) step of the host-driven loop
     alg_bytes_step = (B_RAY * (counts["rays_closest"] + counts["rays_shadow"]) + B_NODE * counts["node_visits"]
@@ -509,7 +522,7 @@ def run_ours(args):
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:
         cpu = cpu_baseline(scene, st, args.cpu_seconds,
-                           frame_nodes_per_sample=counts["node_visits"] / max(1, counts["samples"]))
+                           frame_nodes_per_sample=ref_counts["node_visits"] / max(1, ref_counts["samples"]))
     if relmse is not None:
         # time to reach this relMSE: every arm computes the same per-sample values,
         # so each needs the frame's samples, at its own rate
@@ -795,10 +808,7 @@ def batch_line(args, rank, world, local, dist):
         tuned = host.autotune(probe)
         mode = N.RENDERER_WAVEFRONT_GRAPH if tuned["renderer"] == N.RENDERER_WAVEFRONT_GRAPH else N.RENDERER_WAVEFRONT
         host.set_renderer(mode)
-    host.set_counting(True)
-    host.render_batch_device(items(0), ptrs, stream)
-    counts = host.stats()
-    host.set_counting(False)
+    _, counts = counting_passes(host, lambda: host.render_batch_device(items(0), ptrs, stream))
     for i in range(args.warmup):
         host.render_batch_device(items(i), ptrs, stream)
     torch.cuda.synchronize()

@@ -106,6 +106,7 @@ struct Ctx {
     unsigned long long* stats = nullptr;       /* head + 128 */
     void* io = nullptr; size_t io_bytes = 0;   /* device staging for host-pointer calls */
     bool counting = false;
+    bool count_traced = false;                 /* counting: the rays of a run that does not count (rt_debug_count_traced) */
     cudaStream_t call_stream = nullptr;        /* the stream of the call that has begun */
     bool unfinished = false;                   /* a call has begun and not finished (begin_call) */
     bool late_ms = false;                      /* events[0..1] hold the last round's time (finish_call) */
@@ -1181,7 +1182,7 @@ void particle_wavefront(Ctx* c, const RtParams& P, int64_t first, int64_t count,
     W.shadow_base = 2 * slots;
     W.refill = c->wf_refill;
     W.iter_cap = c->wf_iter_cap;
-    W.mis_any = c->counting ? 0 : 1;
+    W.mis_any = c->counting && !c->count_traced ? 0 : 1;
     W.dense_sort = 1;
     WfMode m;
     m.particle = true;
@@ -1380,7 +1381,7 @@ struct WfJobIn {
  * condition when no path is left.  Rebuilt when the path state moves or the
  * counting mode changes. */
 void ensure_wf_graph(Ctx* c, const WfState& W, const WfMode& m) {
-    const uint64_t key = (c->wf_generation << 32) ^ ((uint64_t)m.wide << 63) ^ ((uint64_t)m.general << 62) ^ ((uint64_t)m.grow << 61) ^ ((uint64_t)W.slots << 10) ^ ((uint64_t)m.deep << 9) ^
+    const uint64_t key = (c->wf_generation << 32) ^ ((uint64_t)m.wide << 63) ^ ((uint64_t)m.general << 62) ^ ((uint64_t)m.grow << 61) ^ ((uint64_t)W.mis_any << 60) ^ ((uint64_t)W.slots << 10) ^ ((uint64_t)m.deep << 9) ^
                          ((uint64_t)(uint32_t)W.iter_cap * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)(uint32_t)W.finish_max * 0xC2B2AE3D27D4EB4Full) ^
                          ((uint64_t)m.sort << 8) ^ ((uint64_t)m.particle << 7) ^ ((uint64_t)W.refill << 2) ^
                          ((uint64_t)m.vol << 1) ^ (c->counting ? 1u : 0u);
@@ -1489,7 +1490,7 @@ void wavefront_run(Ctx* c, const std::vector<WfJobIn>& jobs, cudaStream_t s, boo
         W.shadow_base = 2 * slots;
         W.refill = c->wf_refill;
         W.iter_cap = c->wf_iter_cap;
-        W.mis_any = c->counting ? 0 : 1;
+        W.mis_any = c->counting && !c->count_traced ? 0 : 1;
         /* vol_path's shade runs slower from slots walked in index order (C3: 115.3 -> 112.5 M samples/s) */
         W.dense_sort = mode.vol ? 0 : 1;
         /* one pass over the round's samples: start every slot, bounce until no path is left */
@@ -2118,6 +2119,16 @@ int rt_debug_set_finish(void* ctx, int paths) {
     Ctx* c = (Ctx*)ctx;
     if (!c || paths < -1) return RT_ERR_INVALID_ARG;
     c->wf_finish = paths;
+    return RT_OK;
+}
+/* hook (not part of radiantium.h): what a counting wavefront run counts.  0: the
+ * reference's rays; 1: the rays that a run without counting traces, whose MIS
+ * rays of infinite lights are any-hit rays, and only where they carry a term.
+ * Films are the same. */
+int rt_debug_count_traced(void* ctx, int on) {
+    Ctx* c = (Ctx*)ctx;
+    if (!c) return RT_ERR_INVALID_ARG;
+    c->count_traced = on != 0;
     return RT_OK;
 }
 /* test hook: primitive count from which upload_scene builds trees on the GPU */

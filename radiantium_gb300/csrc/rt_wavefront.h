@@ -82,7 +82,7 @@ struct WfState {
     int32_t refill;          /* idle lanes of a trace warp before it fetches new rays */
     int32_t iter_cap;        /* bounce iterations of one round before the run gives up (WF_ITER_CAP) */
     int32_t finish_max;      /* active slots from which rt_wf_finish ends the round; 0: the loop runs to its end */
-    int32_t mis_any;         /* infinite lights' MIS rays are any-hit rays (not while counting rays) */
+    int32_t mis_any;         /* infinite lights' MIS rays are any-hit rays (not while counting the reference's rays) */
     int32_t dense_sort;      /* the shade-key sort may walk the slots in index order (not for vol_path) */
     WfCounters* ctr;
     const WfJob* jobs;

@@ -60,6 +60,12 @@ class Device:
     def set_counting(self, on: bool):
         self._check(self.lib.rt_set_counting(self.h, 1 if on else 0))
 
+    def count_traced(self, on: bool):
+        """What a counting wavefront run counts: the rays that a run without counting traces (on),
+        or the reference's (off, the default), which also traces an infinite light's MIS ray to its
+        closest hit and where it can carry nothing."""
+        self._check(self.lib.rt_debug_count_traced(self.h, 1 if on else 0))
+
     def set_renderer(self, mode: int):
         """N.RENDERER_AUTO / RENDERER_MEGAKERNEL / RENDERER_WAVEFRONT"""
         self._check(self.lib.rt_set_renderer(self.h, mode))
