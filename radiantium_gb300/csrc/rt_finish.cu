@@ -155,9 +155,18 @@ struct FinishGrids {
 
 }  // namespace
 
+static const FinishGrids& finish_grids() {
+    static const FinishGrids grids;
+    return grids;
+}
+
+int rt_wf_finish_lanes(bool wide, bool grow) {
+    return finish_grids().blocks[kFinishPath][wide ? 1 : (grow ? 2 : 0)] * WF_FINISH_BLOCK;
+}
+
 cudaError_t rt_wf_finish(const WfState& W, uint32_t* status, unsigned long long* stats, cudaStream_t s, int pass, bool vol,
                          bool particle, bool wide, bool grow) {
-    static const FinishGrids grids;
+    const FinishGrids& grids = finish_grids();
     cudaError_t e = rt_wf_phase(W, s);
     if (e != cudaSuccess) return e;
     const int k = particle ? kFinishParticle : (vol ? kFinishVol : kFinishPath), w = wide ? 1 : (grow ? 2 : 0);

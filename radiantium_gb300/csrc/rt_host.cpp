@@ -1067,10 +1067,18 @@ int finish_at(const Ctx* c, const WfMode& m) {
     return m.vol || m.particle ? 65536 : 8192;
 }
 /* Paths up to which a round has no loop at all, where the loop would make a
- * handful of iterations of a few launches and a wait each: one material type,
- * 64 Ki Cornell samples 0.52 ms with the loop and 0.39 without. */
+ * handful of iterations of a few launches and a wait each: for a path scene of
+ * one material type, one path for every lane of rt_wf_finish's resident grid
+ * (76 Ki on 152 SMs).  Beyond that a lane runs a second path after its first.
+ * 1-spp films, ms with the loop / without, at 16 / 48 / 76 / 80 / 96 / 128 Ki
+ * samples: Cornell box 0.46 / 0.29, 0.49 / 0.33, 0.51 / 0.39, 0.52 / 0.46, 0.53 /
+ * 0.53, 0.58 / 0.62; the box in rough plastic 0.47 / 0.42, 0.54 / 0.44, 0.56 /
+ * 0.53, 0.57 / 0.62, 0.59 / 0.73, 0.63 / 0.88; the box with a displaced sphere of
+ * 49 k triangles 0.87 / 0.50, 0.96 / 0.62, 1.00 / 0.69, 1.02 / 0.82, 1.05 / 0.93,
+ * 1.15 / 1.09. */
 int whole_round(const Ctx* c, const WfMode& m) {
-    return m.one_type && c->wf_finish < 0 ? 65536 : finish_at(c, m);
+    if (c->wf_finish >= 0 || !m.one_type || m.vol) return finish_at(c, m);
+    return std::max(finish_at(c, m), rt_wf_finish_lanes(m.wide, m.grow));
 }
 
 /* One round of a wavefront run over the jobs already in c->d_jobs: every slot

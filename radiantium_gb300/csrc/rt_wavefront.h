@@ -168,5 +168,7 @@ cudaError_t rt_wf_phase(const WfState& W, cudaStream_t s);
  * adjoint's replay, for counting or for scenes with general_trees. */
 cudaError_t rt_wf_finish(const WfState& W, uint32_t* status, unsigned long long* stats, cudaStream_t s, int pass,
                          bool vol, bool particle, bool wide, bool grow);
+/* the lanes of rt_wf_finish's grid for `path`: every SM filled once */
+int rt_wf_finish_lanes(bool wide, bool grow);
 
 #endif
