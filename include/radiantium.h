@@ -369,8 +369,9 @@ int rt_set_renderer(void* ctx, int mode);
  * the same trees collapsed 8-wide with quantised child boxes read as six
  * 16-byte loads per node, children visited near to far.  It finds the same
  * closest primitive except where two candidates have exactly the same t
- * (flagged RT_HIT_TIE by either traversal) or where the reference's own slab
- * test misses a box at rounding scale; node-visit counters count wide nodes.
+ * (flagged RT_HIT_TIE by either traversal), where the reference's own slab
+ * test misses a box at rounding scale, or where a ray's finite max_t grows (its
+ * first hit lies in an instance, at a world distance beyond max_t); node-visit counters count wide nodes.
  * A scene whose wide trees could overflow the 64-entry stack (or whose binary
  * trees are deeper than 65 levels) renders with the exact traversal;
  * rt_get_traversal reports what the next call will use. */

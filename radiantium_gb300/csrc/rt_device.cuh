@@ -606,7 +606,8 @@ DF bool NearTie(float a, float b) {
  * interval is widened by 2^-20 of its ends, so a child box is never missed
  * where its exact box is hit: the fast traversal visits a superset of the
  * boxes the reference's slab test accepts and finds every primitive hit the
- * reference finds.  Hit children are ordered near to far by a sorting network
+ * reference finds (but for boxes beyond a finite MaxT that grows later, see
+ * VisitNodeFast).  Hit children are ordered near to far by a sorting network
  * over 32-bit keys (entry distance with its low three bits replaced by the
  * child's index, which rounds the distance down); the nearest is descended
  * into and the others are pushed far-first with the rounded-down distance,

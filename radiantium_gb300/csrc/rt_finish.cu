@@ -10,9 +10,10 @@
  * traversal are the loop's own (rt_wavefront.cuh), so every sample has the same
  * bits; a finished path's slot takes the next camera sample here too.
  *
- * Measured against the loop running to its end (ms): volume 16 spp 26.9 -> 20.6
+ * Measured against the loop running to its end (ms): volume 16 spp 26.4 -> 20.1
  * (its loop made about 90 iterations of under 64 Ki paths, each as long as its
- * longest ray), light tracer 15.7 -> 13.0, gradient step 5.26 -> 5.04.
+ * longest ray), light tracer 15.5 -> 13.1, gradient step 5.2 -> 4.9, 256 x 256
+ * preview 0.53 -> 0.36, batch of twelve scenes 34.3 -> 33.3.
  */
 #include "rt_wavefront.cuh"
 
@@ -20,9 +21,12 @@ namespace {
 
 enum FinishKind { kFinishPath, kFinishVol, kFinishParticle };
 
-/* resident blocks per SM.  Path: a whole round of 64 Ki Cornell samples takes 0.39
- * ms at 4 and 0.48 at 3 (more warps); vol_path and the light tracer, which take
- * over long tails: 20.5 / 13.4 ms at 4, 20.4 / 13.3 at 3, 20.6 / 13.3 at 2. */
+/* resident blocks per SM.  Path, whole rounds, ms at 3 / 4 / 5: Cornell box 16 Ki
+ * samples 0.31 / 0.29 / 0.36, 64 Ki 0.48 / 0.36 / 0.42, 96 Ki 0.65 / 0.54 / 0.54; in
+ * rough plastic 0.42 / 0.42 / 0.52, 0.65 / 0.48 / 0.57, 0.92 / 0.73 / 0.74; with a
+ * displaced sphere 0.53 / 0.51 / 0.57, 0.85 / 0.66 / 0.73, 1.07 / 0.93 / 0.91.
+ * vol_path and the light tracer, which take over long tails: 20.5 / 13.4 ms at 4,
+ * 20.4 / 13.3 at 3, 20.6 / 13.3 at 2. */
 #ifndef RT_FINISH_BLOCKS
 #define RT_FINISH_BLOCKS 3
 #endif

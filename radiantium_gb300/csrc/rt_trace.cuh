@@ -61,7 +61,10 @@ template <> struct TraceStack<true> {
  * (5-level tree) at 12 / 16 / 20 / 24: 3.70 / 3.58 / 3.53 / 3.52, against 3.73
  * with up to three nodes and one leaf per step; of a 16-spp pass over the
  * 64 x 200 k-triangle instances at 4 / 8 / 12 / 14 / 16 / 20: 82.7 / 76.3 /
- * 73.1 / 72.8 / 72.7 / 75.3, against 79.6 with up to five nodes per step. */
+ * 73.1 / 72.8 / 72.7 / 75.3, against 79.6 with up to five nodes per step.
+ * With the short node visit: Cornell frame at 12 / 18 / 20 / 22 / 24: 2.83 / 2.62 /
+ * 2.57 / 2.52 / 2.50, the instances at 12 / 14 / 16: 48.7 / 48.1 / 47.8; whole calls
+ * at 24 and 16 take 0.4 to 1.5 % less, with wide nodes 0.5 % more. */
 #ifndef RT_LEAF_WAIT
 #define RT_LEAF_WAIT 22          /* shallow trees */
 #endif

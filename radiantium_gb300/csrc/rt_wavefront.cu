@@ -6,8 +6,9 @@
  * separate kernels over compacted queues:
  *
  *   k_wf_trace_closest / k_wf_trace_shadow   the queued rays: extension and
- *                MIS rays (closest hit), shadow rays (any hit), each kind in
- *                its own persistent kernel with dynamic ray fetch;
+ *                area lights' MIS rays (closest hit), shadow rays and infinite
+ *                lights' MIS rays (any hit), each kind in its own persistent
+ *                kernel with dynamic ray fetch;
  *   k_wf_sort_count / k_wf_sort_scatter   regroup the active list by shade
  *                key (finished, missed, material type) so that a warp runs
  *                one material's code instead of the union of several;

@@ -296,8 +296,6 @@ DF void finish_path(const WfJob& J, const WfState& W, int slot, C3 rad, unsigned
     o[0] = rad.r; o[1] = rad.g; o[2] = rad.b;
 }
 
-/* one bounce of PathTracer.Mis / NextEventEstimation / OnlySampleBxdf after the
- * extension hit is known (PathTracer.cs:43-270) */
 /* What a path shade leaves for the queues: its shadow ray, whether it
  * queued a MIS ray (in pd_ray_o / pd_ray_d; mis_any: as an any-hit ray) or an
  * extension ray (in ray_o / ray_d), whether the slot stays active, and whether the path is over (the
@@ -427,6 +425,10 @@ DF void schedule_direct(PathOut* o, const WfState& W, const RtSceneView* S, int 
     }
 }
 
+/* Adds the direct term that the slot's previous shade scheduled, then runs one
+ * bounce of PathTracer.Mis / NextEventEstimation / OnlySampleBxdf after its
+ * extension hit (PathTracer.cs:43-270); its rays and what becomes of the slot go
+ * to `o`. */
 template <bool kAdj>
 DF void shade_path(PathOut* o, const WfState& W, int slot, uint32_t* status, unsigned long long* stats, bool counting,
                    int pass, const WfAdjoint& A, float* s_alpha) {
