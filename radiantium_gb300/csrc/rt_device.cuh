@@ -745,8 +745,8 @@ DF bool TraversalBegin(const RtSceneView* S, const Ray& ray, Traversal& T, TravS
  * fast traversal's wide nodes (a visit may push up to seven entries), or in
  * the short form for closest-hit rays whose MaxT may grow (VisitNodeFast's
  * kGrow).  That takes a scene with instances and a finite MaxT that a hit can
- * exceed: a ray batch's, that of vol_path's walks to a light, and the camera's
- * far plane where it does not lie behind the whole scene (RtSceneView::far_cuts).
+ * exceed with a box beyond it: a ray batch's, that of vol_path's walks to a light,
+ * and the camera's far plane where the scene reaches it (RtSceneView::far_cuts).
  * The others keep the plain short form, because the test costs every visit:
  * 16-spp pass over the 64 instances 67.6 -> 68.2 ms, Cornell frame 7.42 -> 7.53,
  * 256 x 256 preview 0.36 -> 0.38; 2 M incoherent rays, which have it, 1.31 -> 1.32. */

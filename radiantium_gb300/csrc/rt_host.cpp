@@ -619,7 +619,6 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
     std::vector<RtLight> lights;
     std::vector<int32_t> infinite;
     std::vector<RtInstance> insts;
-    float inst_terms = 0;                      /* largest sum of the terms of an instance's point, by size */
     auto area_light = [&](int kind, int ref, const rt_group_desc& gd, float area) {
         RtLight L{};
         L.kind = kind; L.ref = ref; L.le[0] = gd.le[0]; L.le[1] = gd.le[1]; L.le[2] = gd.le[2]; L.area = area;
@@ -680,12 +679,6 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
             RtInstance I{};
             rows12(gd.model_to_world, I.m2w); rows12(gd.world_to_model, I.w2m);
             I.root = bvhs[1 + gd.ref];
-            for (int j = 0; j < 3; j++) {
-                float terms = std::fabs(gd.model_to_world[12 + j]);
-                for (int k = 0; k < 3; k++)
-                    terms += std::fabs(gd.model_to_world[4 * k + j]) * std::max(std::fabs(I.root.root_min[k]), std::fabs(I.root.root_max[k]));
-                inst_terms = std::max(inst_terms, terms);
-            }
             int id = (int)prims.size();
             prims.push_back(RtPrim{RT_KIND_INSTANCE, (int)insts.size(), tp.material, -1, tp.med_in, tp.med_out, 0, 0});
             boxes.push_back(xform_box(blas_root[gd.ref], gd.model_to_world));
@@ -856,17 +849,20 @@ void upload_scene(Ctx* c, const rt_scene_desc* d) {
         const float area = std::fabs((cam.max_x - cam.min_x) * (cam.max_y - cam.min_y));
         cam.normalization = 1 / area;
     }
-    /* an instance's hit point lies in the top-level box, which holds its transformed
-     * prototype, so none is further from the camera than the box's farthest corner; the
-     * rounding of the points (of their terms' size) and of the distance is covered amply */
+    /* a top-level box that a camera ray enters at the far plane or behind it lies in the
+     * root's box, so the root's farthest corner is no nearer than the plane (0.999: the
+     * rounding of both distances); a box that is not a number can drop others from a union */
     {
         float corner[3];
         for (int k = 0; k < 3; k++) {
             const float at = cam.camera_to_world[12 + k];
             corner[k] = std::max(std::fabs(v.top.root_min[k] - at), std::fabs(v.top.root_max[k] - at));
         }
-        const float reach = length(f3(corner[0], corner[1], corner[2])) + 1e-5f * inst_terms;
-        v.far_cuts = reach < 0.999f * cam.far_z ? 0 : 1;
+        bool cuts = !(length(f3(corner[0], corner[1], corner[2])) < 0.999f * cam.far_z);
+        if (v.instanced && !cuts)
+            for (const rtb::Box& b : boxes)
+                for (int k = 0; k < 3; k++) cuts = cuts || b.mn[k] != b.mn[k] || b.mx[k] != b.mx[k];
+        v.far_cuts = cuts ? 1 : 0;
     }
     c->d_view = upload(c, std::vector<RtSceneView>{v});
     CK(cudaStreamSynchronize(c->stream));
@@ -1381,7 +1377,7 @@ struct WfJobIn {
     bool wide_ok;          /* its wide trees fit the fast traversal's stack */
     bool general;          /* its trees need the general node visit */
     bool instanced;        /* it has instances */
-    bool far_cuts;         /* its camera's far plane may lie before a hit */
+    bool far_cuts;         /* a top-level box reaches its camera's far plane */
 };
 
 /* The bounce loop as a graph: a while node whose body is one iteration

@@ -184,7 +184,7 @@ struct RtSceneView {
                                  * stack, so every far child is pushed exactly as the reference
                                  * pushes it), or a box has min > max (a negative sphere radius) */
     int32_t instanced;          /* the scene has instances */
-    int32_t far_cuts;           /* an instance's hit may lie beyond the camera's far plane */
+    int32_t far_cuts;           /* a top-level box may lie at the camera's far plane or behind it */
     const float4* wnodes;       /* wide nodes of every tree (RT_WIDE_F4 float4 each) */
     int32_t wide_ok;            /* every wide traversal fits the stack: the fast mode may run */
     int32_t env_alias;          /* infinite lights pick texels from their alias tables */
